@@ -269,19 +269,18 @@ xmpError_t XMPAPI xmpPowmBatchPlanCreate(xmpHandle_t h, const xmpPowmBatchItem_t
     b.blocks = (int)blocks;
     // shrink the window if the tables would exceed the scratch limit
     while (b.cfg.window > 1 &&
-           (size_t)b.blocks * 128 * b.cfg.limbs * 4 * powm_table_entries(b.cfg.window, powm_sliding(b.cfg.tpi, b.cfg.limbs)) >
+           (size_t)b.blocks * 128 * powm_slot_words(b.cfg.tpi, b.cfg.limbs) * 4 *
+               powm_table_entries(b.cfg.window, powm_sliding(b.cfg.tpi, b.cfg.limbs)) >
                scratch_limit(h) / 2)
       b.cfg.window--;
     b.table_offset = bytes;
-    bytes += (size_t)b.blocks * 128 * b.cfg.limbs * 4 * powm_table_entries(b.cfg.window, powm_sliding(b.cfg.tpi, b.cfg.limbs));
+    bytes += (size_t)b.blocks * 128 * powm_slot_words(b.cfg.tpi, b.cfg.limbs) * 4 *
+               powm_table_entries(b.cfg.window, powm_sliding(b.cfg.tpi, b.cfg.limbs));
     bytes = (bytes + 255) & ~(size_t)255;
   }
   // CRT items: window tables for all instances at once, or chunks of what half the scratch limit holds
   for (auto &c : p->crt) {
-    while ((c.chunk = crt_chunk_for(c.cfg, scratch_limit(h) / 2, c.item.count)) == 0) {
-      if (c.cfg.window <= 1) return fail(xmpErrorIncreaseScratchLimit);
-      c.cfg.window--;
-    }
+    if ((c.chunk = crt_fit(c.cfg, scratch_limit(h) / 2, c.item.count)) == 0) return fail(xmpErrorIncreaseScratchLimit);
     c.table_offset = bytes;
     bytes += crt_table_bytes(c.cfg, c.chunk);
     bytes = (bytes + 255) & ~(size_t)255;

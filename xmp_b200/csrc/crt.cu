@@ -14,10 +14,10 @@ std::vector<CrtKernelEntry> &crt_registry() {
 }
 
 #define XMPB_REGISTER_CRT(TPI, L)                                                                 \
-  static void crt_launch_##TPI##_##L(const CrtArgs &a, int grid, cudaStream_t s) {               \
+  static void crt_launch_##TPI##_##L(const CrtArgs &a, int grid, int threads, cudaStream_t s) {  \
     static bool attr = false;                                                                     \
     powm_smem_attr(crt_kernel<TPI, L>, powm_smem_bytes(TPI, L), attr);                            \
-    crt_kernel<TPI, L><<<grid, 128, powm_smem_bytes(TPI, L), s>>>(a);                             \
+    crt_kernel<TPI, L><<<grid, threads, powm_smem_bytes(TPI, L), s>>>(a);                         \
   }                                                                                               \
   static CrtKernelRegistrar crt_reg_##TPI##_##L(TPI, L, crt_launch_##TPI##_##L);
 
@@ -64,22 +64,34 @@ CrtConfig crt_config(uint32_t nlimbs, uint32_t exp_bits, uint32_t count, uint32_
 }
 
 size_t crt_table_bytes(const CrtConfig &c, uint32_t count) {
-  const size_t threads = round_up((uint32_t)std::min<uint64_t>((uint64_t)count * c.tpi * 2, 0xffffff80ull), 128);
-  return threads * (size_t)c.limbs * ((size_t)1 << c.window) * 4;
+  const size_t threads =
+      round_up((uint32_t)std::min<uint64_t>((uint64_t)count * c.tpi * 2, 0xffffff80ull), (uint32_t)c.threads);
+  return threads * (size_t)powm_slot_words(c.tpi, c.limbs) * crt_table_entries(c.tpi, c.limbs, (uint32_t)c.window) * 4;
 }
 
 uint32_t crt_chunk_for(const CrtConfig &c, size_t limit, uint32_t count) {
-  const uint32_t per_block = 128 / (2 * c.tpi);  // a pair of groups per instance
-  const size_t per_inst = (size_t)2 * c.tpi * c.limbs * ((size_t)1 << c.window) * 4;
+  const uint32_t per_block = c.threads / (2 * c.tpi);  // a pair of groups per instance
+  const size_t per_inst = (size_t)2 * c.tpi * powm_slot_words(c.tpi, c.limbs) *
+                          crt_table_entries(c.tpi, c.limbs, (uint32_t)c.window) * 4;
   const uint64_t fit = std::min<uint64_t>(limit / per_inst, (1ull << 31) / (2 * c.tpi)) / per_block * per_block;
   return fit < per_block ? 0u : (uint32_t)std::min<uint64_t>(count, fit);
+}
+
+uint32_t crt_fit(CrtConfig &c, size_t limit, uint32_t count) {
+  uint32_t chunk;
+  while ((chunk = crt_chunk_for(c, limit, count)) == 0) {
+    if (c.window > 1) c.window--;
+    else if (c.threads > 32) c.threads = 32;
+    else return 0;
+  }
+  return chunk;
 }
 
 void crt_launch(const CrtConfig &c, CrtArgs a, uint32_t count, uint32_t chunk, cudaStream_t s) {
   for (uint32_t start = 0; start < count; start += chunk) {
     a.start = start;
     a.count = std::min(chunk, count - start);
-    c.launch(a, grid_for((uint64_t)a.count * c.tpi * 2, 128), s);
+    c.launch(a, grid_for((uint64_t)a.count * c.tpi * 2, c.threads), c.threads, s);
   }
 }
 
@@ -128,12 +140,8 @@ xmpError_t XMPAPI xmpIntegersPowmCRTAsync(xmpHandle_t h, xmpIntegers_t out, cons
   CrtConfig cfg = crt_config(p->nlimbs, std::max(dp->precision, dq->precision), count, h->sm_count);
   if (!cfg.launch) return xmpErrorUnsupported;
   // chunk so the window tables fit the scratch limit; shrink the window when one block does not fit
-  const size_t limit = scratch_limit(h);
-  uint32_t chunk;
-  while ((chunk = crt_chunk_for(cfg, limit, count)) == 0) {
-    if (cfg.window <= 1) return xmpErrorIncreaseScratchLimit;
-    cfg.window--;
-  }
+  const uint32_t chunk = crt_fit(cfg, scratch_limit(h), count);
+  if (chunk == 0) return xmpErrorIncreaseScratchLimit;
   // an output that is also an input is written through the handle's temporary output buffer
   const bool aliased = (out == c || out == p || out == q || out == dp || out == dq || out == qinv);
   OutTarget t;

@@ -33,7 +33,7 @@ struct CrtArgs {
   uint32_t start;   // first op instance of this launch
   uint32_t count;   // op instances in this launch
   uint32_t window;  // fixed-window bits W
-  uint32_t *table;  // per warp: 2^W entries x 32 lanes x L words
+  uint32_t *table;  // per warp: crt_table_entries entries x 32 lanes x powm_slot_words words
 };
 
 // r += x over the group; returns the carry out of the top lane (same in every lane).
@@ -239,6 +239,145 @@ __device__ __forceinline__ uint32_t crt_modulus(const Group<TPI> &G, uint32_t (&
   return np0;
 }
 
+// ---- the same on 52-bit digits (dmont.cuh) -------------------------------------------
+
+// r = the balanced digits of the signed 64-bit digits d (|d| < 2^63, value within +-R / 4).
+template <int TPI, int D>
+__device__ __forceinline__ void dig_balance(const Group<TPI> &G, double (&r)[D], const int64_t (&d)[D]) {
+  uint64_t col[D];
+#pragma unroll
+  for (int j = 0; j < D; j++) col[j] = (uint64_t)d[j];
+  dig_settle<TPI, D>(G, r, col, 0u, 0u);
+}
+
+// The group's 2N canonical digits of add + a * B (B in shared memory, a balanced; add, and the sum, not
+// negative) into out[0 .. 2N).  Rows as in dig_mul without the reduction: column 0 of row i is product
+// digit i once its constant is taken off, and carries into the next column.
+template <int TPI, int D>
+__device__ __forceinline__ void dig_mul_add_wide(const Group<TPI> &G, uint64_t *out, const int64_t (&add)[D],
+                                                 const double (&a)[D], const DigSmem &sm) {
+  constexpr int N = TPI * D;
+  constexpr uint64_t kLo = (uint64_t)kDigLoBits << 52, kHi = (0x467ull << 52) + (1ull << 51);
+  const double *bp = dig_b<TPI, D>(sm);
+  uint64_t col[D + 1], k = kLo;
+#pragma unroll
+  for (int j = 0; j < D; j++) col[j] = (uint64_t)add[j];
+  col[D] = 0;
+#pragma unroll 1
+  for (int i = 0; i < N; i++) {
+    dig_row<D, 0>(col, a, bp[i * (32 / TPI)]);
+    const int64_t v = (int64_t)(col[0] - k);
+    k += kLo + kHi;
+    if (G.lane == 0) out[i] = (uint64_t)v & kDigMask;
+    uint64_t next = 0;
+    if (TPI > 1) {
+      next = __shfl_down_sync(kFull, col[0], 1, TPI);
+      if (G.lane == TPI - 1) next = 0;
+    }
+#pragma unroll
+    for (int j = 0; j < D; j++) col[j] = col[j + 1];
+    col[D] = 0;
+    col[D - 1] += next;
+    if (G.lane == 0) col[0] += (uint64_t)(v >> 52);
+  }
+  int64_t d[D];
+#pragma unroll
+  for (int j = 0; j < D; j++) {
+    const uint64_t p = G.lane * D + j;
+    d[j] = (int64_t)(col[j] - (N - 1 - p) * kLo - (N - p) * kHi);
+  }
+  dig_carry<TPI, D>(G, d);
+#pragma unroll
+  for (int j = 0; j < D; j++) out[N + G.lane * D + j] = (uint64_t)d[j];
+  __syncwarp();
+}
+
+// Steps 1-3 above.  Differences from the limb form: c splits at R = 2^(52N) (its low part balanced, so
+// within R / 2), the two parts' Montgomery forms are added without reducing (below 2N, R >= 16N), and
+// Garner's difference mp - mq goes into the product by qinv signed and unreduced (R >= 16 max(p, q)).
+// R^2 waits in the table's last entry.
+template <int TPI, int L, int D>
+__device__ __forceinline__ void dig_crt_instance(const Group<TPI> &G, const CrtArgs &a, uint32_t i, bool valid,
+                                                 bool second, double *tab, const DigSmem &sm) {
+  static_assert(52 * TPI * D >= 32 * TPI * L + 4, "R >= 16 N");
+  constexpr int N = TPI * D;
+  const ArrayView mv = second ? a.q : a.p, ov = second ? a.p : a.q, ev = second ? a.dq : a.dp;
+  const uint32_t em = in_element(mv, i), W = a.window;
+  const uint32_t nwin = (max(a.dp.nlimbs, a.dq.nlimbs) * 32 + W - 1) / W;
+  double n[D], t[D], acc[D];
+  uint64_t np;
+  dig_load<TPI, D>(G, n, mv.limbs, mv.nlimbs, mv.stride, em);
+  {
+    uint32_t nl[L];
+    load_lane_limbs_at<TPI, L>(nl, mv, em, G.lane, 0);
+    np = dig_neg_inv(nl[0], nl[1]);
+    dig_r2<TPI, L, D>(G, t, nl, n, np, sm);
+  }
+  dig_slot_store<TPI, D>(tab, 1u << W, t);
+  dig_set_b<TPI, D>(G, sm, t);
+  {
+    double one[D];
+#pragma unroll
+    for (int k = 0; k < D; k++) one[k] = (G.lane == 0 && k == 0) ? 1.0 : 0.0;
+    dig_mul<TPI, D>(G, one, one, sm, n, np);
+    dig_slot_store<TPI, D>(tab, 0, one);  // Mont(1)
+  }
+  {
+    const uint32_t ec = in_element(a.c, i);
+    double u[D];
+    dig_mul<TPI, D>(G, t, t, sm, n, np);  // R^3
+    dig_load<TPI, D>(G, acc, a.c.limbs, a.c.nlimbs, a.c.stride, ec);
+    dig_mul<TPI, D>(G, acc, acc, sm, n, np);  // c_lo R
+    dig_set_b<TPI, D>(G, sm, t);
+    dig_load<TPI, D>(G, u, a.c.limbs, a.c.nlimbs, a.c.stride, ec, N);
+    dig_mul<TPI, D>(G, u, u, sm, n, np);  // c_hi R^2
+    int64_t d[D];
+#pragma unroll
+    for (int k = 0; k < D; k++) d[k] = (int64_t)acc[k] + (int64_t)u[k];
+    dig_balance<TPI, D>(G, t, d);
+  }
+  dig_slot_store<TPI, D>(tab, 1, t);
+  const uint32_t ee = in_element(ev, i);
+  dig_fixed_table<TPI, D>(G, acc, t, n, np, W, tab, sm);
+  dig_fixed_scan<TPI, D>(G, acc, ev, ee, nwin, W, n, np, tab, sm);
+#pragma unroll
+  for (int k = 0; k < D; k++) t[k] = (G.lane == 0 && k == 0) ? 1.0 : 0.0;
+  dig_set_b<TPI, D>(G, sm, t);
+  dig_mul<TPI, D>(G, acc, acc, sm, n, np);
+  int64_t mine[D], other[D];
+  dig_canon<TPI, D>(G, mine, acc, n);
+#pragma unroll
+  for (int k = 0; k < D; k++) other[k] = (int64_t)__shfl_xor_sync(kFull, (unsigned long long)mine[k], TPI);
+  dig_slot_load<TPI, D>(tab, 1u << W, t);
+  dig_set_b<TPI, D>(G, sm, t);
+  dig_load<TPI, D>(G, t, a.qinv.limbs, a.qinv.nlimbs, a.qinv.stride, in_element(a.qinv, i));
+  dig_mul<TPI, D>(G, t, t, sm, n, np);  // qinv R
+  dig_set_b<TPI, D>(G, sm, t);
+#pragma unroll
+  for (int k = 0; k < D; k++) mine[k] -= other[k];
+  dig_balance<TPI, D>(G, acc, mine);
+  dig_mul<TPI, D>(G, acc, acc, sm, n, np);  // (mp - mq) qinv mod p
+  dig_canon<TPI, D>(G, mine, acc, n);       // h
+  dig_balance<TPI, D>(G, t, mine);
+  dig_set_b<TPI, D>(G, sm, t);
+  dig_load<TPI, D>(G, t, ov.limbs, ov.nlimbs, ov.stride, in_element(ov, i));
+  // the table is done with: its first 2N digits per group take m = mq + q h
+  uint64_t *st = reinterpret_cast<uint64_t *>(tab) + (size_t)((threadIdx.x & 31) / TPI) * (2 * N);
+  __syncwarp();
+  dig_mul_add_wide<TPI, D>(G, st, other, t, sm);
+  if (valid && !second) {
+    const uint32_t o = out_element(a.out, i);
+    if (o < a.out.count)
+      for (uint32_t g = G.lane; g < div_up(a.out.nlimbs, 4); g += TPI)
+        store_group(a.out.limbs, a.out.nlimbs, a.out.stride, o, g, dig_group(st, 2 * N, g));
+  }
+}
+
+// Words per lane and entries of the window table (the digit form keeps R^2 in one more).
+__host__ __device__ constexpr uint32_t crt_table_entries(int TPI, int L, uint32_t W) {
+  return (1u << W) + (powm_digits(TPI, L) ? 1u : 0u);
+}
+
 // The two exponentiations of an instance run side by side on two adjacent
 // groups of one warp (lanes [0, TPI) of the pair work mod p, lanes
 // [TPI, 2 TPI) mod q), so a batch has twice as many independent groups as
@@ -251,9 +390,9 @@ __device__ __forceinline__ uint32_t crt_modulus(const Group<TPI> &G, uint32_t (&
 // h = (mp - mq mod p) * qinv mod p and m = mq + q h, which it stores; the
 // second group's mirror image is discarded.
 template <int TPI, int L>
-__global__ void __launch_bounds__(128) crt_kernel(CrtArgs a) {
+__global__ void __launch_bounds__(128, powm_min_blocks(TPI, L)) crt_kernel(CrtArgs a) {
   static_assert(TPI <= 16, "both groups of a pair sit in one warp");
-  const SqrSmem sm = powm_smem_setup<TPI, L>();
+  const PowmSmem psm = powm_smem_setup<TPI, L>();
   Group<TPI> G;
   const uint32_t gtid = blockIdx.x * blockDim.x + threadIdx.x;
   const uint32_t local = gtid / (2 * TPI);
@@ -261,7 +400,14 @@ __global__ void __launch_bounds__(128) crt_kernel(CrtArgs a) {
   const bool valid = local < a.count;
   // pairs past the end run a copy of the last instance so every shuffle sees a full warp
   const uint32_t i = a.start + (valid ? local : a.count - 1);
-  uint32_t *slot = a.table + (size_t)(gtid >> 5) * ((size_t)32 * L * (1u << a.window)) + (size_t)(threadIdx.x & 31) * L;
+  uint32_t *table = a.table + (size_t)(gtid >> 5) * ((size_t)32 * powm_slot_words(TPI, L) *
+                                                     crt_table_entries(TPI, L, a.window));
+  if constexpr (powm_digits(TPI, L) > 0) {
+    dig_crt_instance<TPI, L, powm_digits(TPI, L)>(G, a, i, valid, second, reinterpret_cast<double *>(table), psm.dig);
+    return;
+  } else {
+  const SqrSmem &sm = psm.sqr;
+  uint32_t *const slot = table + (size_t)(threadIdx.x & 31) * L;
   const ArrayView mv = second ? a.q : a.p, ov = second ? a.p : a.q, ev = second ? a.dq : a.dp;
   const uint32_t em = in_element(mv, i);
   const uint32_t nbits = max(a.dp.nlimbs, a.dq.nlimbs) * 32;
@@ -318,6 +464,7 @@ __global__ void __launch_bounds__(128) crt_kernel(CrtArgs a) {
       store_lane_limbs_at<TPI, L>(lo, a.out, o, G.lane, 0);
       store_lane_limbs_at<TPI, L>(hi, a.out, o, G.lane, n_limbs);
     }
+  }
   }
 }
 

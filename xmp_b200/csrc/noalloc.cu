@@ -25,6 +25,7 @@
 // caller makes current, gets its own lookup rather than a stale address.
 // Make the first call in a context before any stream capture.
 #include "powm.h"
+#include <algorithm>
 #include <cuda.h>
 #include <mutex>
 
@@ -122,9 +123,16 @@ extern "C" xmpError_t XMPAPI xmpIntegersPowmNoAlloc(cudaStream_t stream, uint32_
   // far larger than the fixed scratch.
   PowmConfig cfg = powm_default_config(nlimbs, exp_precision, count, xmpAlgorithmDefault, (uint32_t)sms);
   if (cfg.dist != kDistLanes || !powm_config_valid(cfg, nlimbs)) return xmpErrorUnsupported;
-  // Shrink the window until the tables fit the fixed array; beyond that the batch is too large.
+  // Shrink the window until the tables fit the fixed array.  The documented limit on the batch is two
+  // entries per instance in limbs; a kernel whose entries are larger (digits) takes a batch up to that
+  // limit in more than one launch.
+  const uint64_t cta = 128 / cfg.tpi;
+  if (round_up(count, cta) * (uint64_t)cfg.tpi * cfg.limbs * 2 * 4 > kNoAllocScratchBytes)
+    return xmpErrorIncreaseScratchLimit;
   while (powm_table_bytes(cfg, nlimbs, count) > kNoAllocScratchBytes && cfg.window > 1) cfg.window--;
-  if (powm_table_bytes(cfg, nlimbs, count) > kNoAllocScratchBytes) return xmpErrorIncreaseScratchLimit;
+  uint32_t chunk = count;
+  if (powm_table_bytes(cfg, nlimbs, count) > kNoAllocScratchBytes)
+    chunk = (uint32_t)(kNoAllocScratchBytes / powm_table_bytes(cfg, nlimbs, (uint32_t)cta) * cta);
   const PowmKernelEntry *k = powm_find(cfg.tpi, cfg.limbs);
   if (!k) return xmpErrorUnsupported;
 
@@ -137,10 +145,12 @@ extern "C" xmpError_t XMPAPI xmpIntegersPowmNoAlloc(cudaStream_t stream, uint32_
   a.exp = ArrayView{const_cast<uint32_t *>(exp), exp_precision / 32, stride, count, nullptr, 0};
   a.mod = ArrayView{const_cast<uint32_t *>(mod), nlimbs, stride, count, nullptr, 0};
   a.out = OutView{out, nlimbs, stride, count, nullptr};
-  a.start = 0;
-  a.count = count;
   a.window = (uint32_t)cfg.window;
   a.table = (uint32_t *)scratch;
-  k->launch(a, grid_for((uint64_t)count * cfg.tpi, 128), stream);
+  for (uint32_t start = 0; start < count; start += chunk) {
+    a.start = start;
+    a.count = std::min(chunk, count - start);
+    k->launch(a, grid_for((uint64_t)a.count * cfg.tpi, 128), 128, stream);
+  }
   return cudaPeekAtLastError() == cudaSuccess ? xmpErrorSuccess : xmpErrorCuda;
 }

@@ -108,15 +108,16 @@ PowmConfig powm_default_config(uint32_t nlimbs, uint32_t exp_bits, uint32_t coun
   return best;
 }
 
-size_t powm_table_bytes(const PowmConfig &cfg, uint32_t nlimbs, uint32_t count) {
+size_t powm_table_bytes(const PowmConfig &cfg, uint32_t nlimbs, uint32_t count, uint32_t cta_threads) {
   if (cfg.dist == kDistCta) return 0;  // the table is in shared memory
   if (cfg.dist == kDistDigit) {
     // table + N, x, b, m, r, r2 working arrays, all nlimbs+2 words per instance
     size_t words = ((size_t)1 << cfg.window) * nlimbs + 6 * ((size_t)nlimbs + 2);
     return words * 4 * round_up(count, 128);
   }
-  size_t threads = round_up((uint32_t)std::min<uint64_t>((uint64_t)count * cfg.tpi, 0xffffff80ull), 128);
-  return threads * (size_t)cfg.limbs * powm_table_entries(cfg.window, powm_sliding(cfg.tpi, cfg.limbs)) * 4;
+  size_t threads = round_up((uint32_t)std::min<uint64_t>((uint64_t)count * cfg.tpi, 0xffffff80ull), cta_threads);
+  return threads * (size_t)powm_slot_words(cfg.tpi, cfg.limbs) *
+         powm_table_entries(cfg.window, powm_sliding(cfg.tpi, cfg.limbs)) * 4;
 }
 
 xmpError_t powm_run(xmpHandle_t h, const PowmConfig &cfg0, const OutView &out, const ArrayView &base,
@@ -139,21 +140,30 @@ xmpError_t powm_run(xmpHandle_t h, const PowmConfig &cfg0, const OutView &out, c
   const PowmKernelEntry *k = powm_find(cfg.tpi, cfg.limbs);
   if (!k) return xmpErrorUnsupported;
   size_t limit = scratch_limit(h);
-  // Chunk so the window tables fit; shrink the window if even one block of instances does not fit.
+  // Chunk so the window tables fit; shrink the window if even one CTA's instances do not fit, then the CTA
+  // to one warp.
+  int threads = 128;
   uint32_t per_block = 128 / cfg.tpi;
   uint32_t chunk = count;
   while (true) {
-    size_t per_inst = (size_t)cfg.tpi * cfg.limbs * powm_table_entries(cfg.window, powm_sliding(cfg.tpi, cfg.limbs)) * 4;
+    size_t per_inst = (size_t)cfg.tpi * powm_slot_words(cfg.tpi, cfg.limbs) *
+                      powm_table_entries(cfg.window, powm_sliding(cfg.tpi, cfg.limbs)) * 4;
     uint64_t fit = limit / per_inst;
     fit = fit / per_block * per_block;
     if (fit >= per_block) {
       chunk = (uint32_t)std::min<uint64_t>(count, fit);
       break;
     }
-    if (cfg.window <= 1) return xmpErrorIncreaseScratchLimit;
-    cfg.window--;
+    if (cfg.window > 1) {
+      cfg.window--;
+    } else if (threads > 32) {
+      threads = 32;
+      per_block = 32 / cfg.tpi;
+    } else {
+      return xmpErrorIncreaseScratchLimit;
+    }
   }
-  xmpError_t e = ensure_scratch(h, powm_table_bytes(cfg, mod.nlimbs, chunk));
+  xmpError_t e = ensure_scratch(h, powm_table_bytes(cfg, mod.nlimbs, chunk, threads));
   if (e != xmpErrorSuccess) return e;
   PowmArgs a;
   a.base = base;
@@ -165,8 +175,7 @@ xmpError_t powm_run(xmpHandle_t h, const PowmConfig &cfg0, const OutView &out, c
   for (uint32_t start = 0; start < count; start += chunk) {
     a.start = start;
     a.count = std::min(chunk, count - start);
-    int grid = grid_for((uint64_t)a.count * cfg.tpi, 128);
-    k->launch(a, grid, h->stream);
+    k->launch(a, grid_for((uint64_t)a.count * cfg.tpi, threads), threads, h->stream);
   }
   return check_cuda();
 }

@@ -24,7 +24,8 @@ bool powm_cta_launch(uint32_t limbs, bool ct, const PowmArgs &a, uint32_t count,
 // Whether a batch this small runs faster one instance per CTA than on the lane kernels.
 bool powm_cta_preferred(uint32_t nlimbs, uint32_t count, uint32_t sm_count);
 
-typedef void (*PowmLauncher)(const PowmArgs &args, int grid, cudaStream_t stream);
+// Grid of CTAs of `threads` threads (128, or 32 where the scratch limit holds no more window tables).
+typedef void (*PowmLauncher)(const PowmArgs &args, int grid, int threads, cudaStream_t stream);
 typedef void (*PowmBatchLauncher)(const PowmBatchArgs &args, int grid, cudaStream_t stream);
 
 struct PowmKernelEntry {
@@ -36,7 +37,7 @@ struct PowmKernelEntry {
   const void *batch_fn;
   PowmLauncher launch_r2;
   PowmLauncher launch_ct;  // constant schedule (fixed window over the exponent precision), for secret exponents
-  uint32_t smem;           // dynamic shared memory per 128-thread CTA (the four-lane squaring's blocks)
+  uint32_t smem;           // dynamic shared memory per 128-thread CTA (the digit kernels' operand B)
 };
 
 std::vector<PowmKernelEntry> &powm_registry();
@@ -58,29 +59,29 @@ inline void powm_smem_attr(F *fn, uint32_t bytes, bool &done) {
   }
 }
 
-#define XMPB_REGISTER_POWM(TPI, L)                                                                   \
-  static void powm_launch_##TPI##_##L(const PowmArgs &a, int grid, cudaStream_t s) {                \
-    static bool attr = false;                                                                         \
-    powm_smem_attr(powm_kernel<TPI, L>, powm_smem_bytes(TPI, L), attr);                              \
-    powm_kernel<TPI, L><<<grid, 128, powm_smem_bytes(TPI, L), s>>>(a);                              \
-  }                                                                                                   \
-  static void powm_launch_batch_##TPI##_##L(const PowmBatchArgs &a, int grid, cudaStream_t s) {     \
-    static bool attr = false;                                                                         \
-    powm_smem_attr(powm_batch_kernel<TPI, L>, powm_smem_bytes(TPI, L), attr);                        \
-    powm_batch_kernel<TPI, L><<<grid, 128, powm_smem_bytes(TPI, L), s>>>(a);                        \
-  }                                                                                                   \
-  static void powm_launch_r2_##TPI##_##L(const PowmArgs &a, int grid, cudaStream_t s) {             \
-    r2_kernel<TPI, L><<<grid, 128, 0, s>>>(a);                                                       \
-  }                                                                                                   \
-  static void powm_launch_ct_##TPI##_##L(const PowmArgs &a, int grid, cudaStream_t s) {             \
-    static bool attr = false;                                                                         \
-    powm_smem_attr(powm_kernel<TPI, L, true>, powm_smem_bytes(TPI, L), attr);                        \
-    powm_kernel<TPI, L, true><<<grid, 128, powm_smem_bytes(TPI, L), s>>>(a);                        \
-  }                                                                                                   \
-  static PowmKernelRegistrar powm_reg_##TPI##_##L(TPI, L, powm_launch_##TPI##_##L,                  \
-                                                  (const void *)powm_kernel<TPI, L>,                 \
-                                                  powm_launch_batch_##TPI##_##L,                     \
-                                                  (const void *)powm_batch_kernel<TPI, L>,           \
+#define XMPB_REGISTER_POWM(TPI, L)                                                                       \
+  static void powm_launch_##TPI##_##L(const PowmArgs &a, int grid, int threads, cudaStream_t s) {        \
+    static bool attr = false;                                                                            \
+    powm_smem_attr(powm_kernel<TPI, L>, powm_smem_bytes(TPI, L), attr);                                  \
+    powm_kernel<TPI, L><<<grid, threads, powm_smem_bytes(TPI, L), s>>>(a);                               \
+  }                                                                                                      \
+  static void powm_launch_batch_##TPI##_##L(const PowmBatchArgs &a, int grid, cudaStream_t s) {          \
+    static bool attr = false;                                                                            \
+    powm_smem_attr(powm_batch_kernel<TPI, L>, powm_smem_bytes(TPI, L), attr);                            \
+    powm_batch_kernel<TPI, L><<<grid, 128, powm_smem_bytes(TPI, L), s>>>(a);                             \
+  }                                                                                                      \
+  static void powm_launch_r2_##TPI##_##L(const PowmArgs &a, int grid, int threads, cudaStream_t s) {     \
+    r2_kernel<TPI, L><<<grid, threads, powm_smem_bytes(TPI, L), s>>>(a);                                 \
+  }                                                                                                      \
+  static void powm_launch_ct_##TPI##_##L(const PowmArgs &a, int grid, int threads, cudaStream_t s) {     \
+    static bool attr = false;                                                                            \
+    powm_smem_attr(powm_kernel<TPI, L, true>, powm_smem_bytes(TPI, L), attr);                            \
+    powm_kernel<TPI, L, true><<<grid, threads, powm_smem_bytes(TPI, L), s>>>(a);                         \
+  }                                                                                                      \
+  static PowmKernelRegistrar powm_reg_##TPI##_##L(TPI, L, powm_launch_##TPI##_##L,                       \
+                                                  (const void *)powm_kernel<TPI, L>,                     \
+                                                  powm_launch_batch_##TPI##_##L,                         \
+                                                  (const void *)powm_batch_kernel<TPI, L>,               \
                                                   powm_launch_r2_##TPI##_##L, powm_launch_ct_##TPI##_##L, \
                                                   powm_smem_bytes(TPI, L));
 
@@ -104,8 +105,8 @@ bool powm_config_valid(const PowmConfig &c, uint32_t nlimbs);
 xmpError_t powm_run(xmpHandle_t h, const PowmConfig &cfg, const OutView &out, const ArrayView &base,
                     const ArrayView &exp, const ArrayView &mod, uint32_t count);
 
-// Scratch bytes one launch of `count` instances needs.
-size_t powm_table_bytes(const PowmConfig &cfg, uint32_t nlimbs, uint32_t count);
+// Scratch bytes one launch of `count` instances needs (register kernels: CTAs of `cta_threads`).
+size_t powm_table_bytes(const PowmConfig &cfg, uint32_t nlimbs, uint32_t count, uint32_t cta_threads = 128);
 
 // Digit-serial kernel launcher (any precision).
 xmpError_t powm_digit_run(xmpHandle_t h, const PowmConfig &cfg, const OutView &out, const ArrayView &base,

@@ -39,6 +39,7 @@
 // does not change the result.
 #pragma once
 #include "internal.h"
+#include "dmont.cuh"
 #include "mont.cuh"
 #include "sqr.cuh"
 
@@ -52,29 +53,24 @@ struct PowmArgs {
   uint32_t start;   // first op instance of this launch
   uint32_t count;   // op instances in this launch
   uint32_t window;  // window bits W, 1..7
-  uint32_t *table;  // scratch: (launch threads / 32) * 32 * L * powm_table_entries(W, powm_sliding(TPI, L)) words
+  uint32_t *table;  // scratch: per warp 32 * powm_slot_words(TPI, L) * powm_table_entries(W, powm_sliding(TPI, L)) words
 };
 
 // Exponentiation method of the register kernel with TPI lanes x L limbs:
 // sliding window (true) or fixed window (false).  Per shape, from a B200
-// sweep of every registered kernel with both methods (exponents of
-// min(precision, 2048) bits; a batch of 75,776 / TPI instances and a single
-// instance): the sliding window does ~3-4% fewer Montgomery multiplies but
-// adds per-step control, so it is taken where it is faster at the batch and
-// the batch and single-instance gains together are positive -- the 16-limb
-// shapes and a few mid-size ones (2048 bits, 4 x 16: +0.8%; 3072 bits,
-// 16 x 6: +4.8%; 1280 bits, 8 x 5: +8.1%).  It loses at 12 limbs per lane
-// (-7 to -9%: the compiler's schedule of the multiply inside the sliding loop
-// is worse there) and at small precisions, where the control is a larger
-// share of a step.
+// sweep of every registered kernel with both methods (a batch that fills the
+// GPU, fractions of it and a single instance).  The sliding window does ~3-4%
+// fewer Montgomery multiplies but adds per-step control.  Digit kernels: it
+// wins except on one lane and on two lanes up to 8 limbs, where the instances
+// of a warp read their table entries from as many places and the control is a
+// larger share (2048 bits, 4 x 16: 21.8 against 22.4 ms; 256 bits, 1 x 8: 1.01
+// against 0.85 ms; 2 x 8: 3.73 against 3.58).  Limb kernels (below six limbs a
+// lane): where it was faster at the batch and the batch and single-instance
+// gains together were positive (1280 bits, 8 x 5: +8.1%; 16 x 4: +3.3%).
 __host__ __device__ constexpr bool powm_sliding(int TPI, int L) {
-  return !powm_sqr(TPI, L) && (
-         (TPI == 1 && (L == 24 || L == 32)) ||
-         (TPI == 2 && (L == 8 || L == 16)) ||
-         (TPI == 4 && (L == 5 || L == 6 || L == 16)) ||
-         (TPI == 8 && (L == 4 || L == 5 || L == 6 || L == 16)) ||
-         (TPI == 16 && (L == 2 || L == 4 || L == 6 || L == 16)) ||
-         (TPI == 32 && (L == 8 || L == 16)));
+  return powm_digits(TPI, L) ? TPI >= 4 || (TPI == 2 && L >= 12) || L >= 24
+                             : (TPI == 4 && L == 5) || (TPI == 8 && (L == 4 || L == 5)) ||
+                                   (TPI == 16 && (L == 2 || L == 4));
 }
 
 // Window-table entries for window bits W.  Sliding: slot 0 holds Mont(1) and
@@ -243,16 +239,211 @@ __device__ __forceinline__ uint32_t exp_bitlen(const Group<TPI> &G, const ArrayV
   return G.seg_max(bl);
 }
 
+// ---- exponentiation on 52-bit digits (dmont.cuh) ------------------------------------
+
+// Window table of one warp: entry e of this lane's digits.  From four lanes an instance on, digit j of the
+// 32 lanes lies together (the lanes of an instance read whole 32-byte sectors); below that a lane's digits do.
+template <int TPI, int D>
+__device__ __forceinline__ void dig_slot_store(double *tab, uint32_t e, const double (&x)[D]) {
+  const uint32_t l = threadIdx.x & 31;
+  if constexpr (TPI >= 4) {
+    double *p = tab + (size_t)e * 32 * D + l;
+#pragma unroll
+    for (int j = 0; j < D; j++) p[j * 32] = x[j];
+  } else if constexpr (D % 2 == 0) {
+    double2 *p = reinterpret_cast<double2 *>(tab + ((size_t)e * 32 + l) * D);
+#pragma unroll
+    for (int j = 0; j < D / 2; j++) p[j] = make_double2(x[2 * j], x[2 * j + 1]);
+  } else {
+    double *p = tab + ((size_t)e * 32 + l) * D;
+#pragma unroll
+    for (int j = 0; j < D; j++) p[j] = x[j];
+  }
+}
+template <int TPI, int D>
+__device__ __forceinline__ void dig_slot_load(const double *tab, uint32_t e, double (&x)[D]) {
+  const uint32_t l = threadIdx.x & 31;
+  if constexpr (TPI >= 4) {
+    const double *p = tab + (size_t)e * 32 * D + l;
+#pragma unroll
+    for (int j = 0; j < D; j++) x[j] = p[j * 32];
+  } else if constexpr (D % 2 == 0) {
+    const double2 *p = reinterpret_cast<const double2 *>(tab + ((size_t)e * 32 + l) * D);
+#pragma unroll
+    for (int j = 0; j < D / 2; j++) {
+      const double2 v = p[j];
+      x[2 * j] = v.x;
+      x[2 * j + 1] = v.y;
+    }
+  } else {
+    const double *p = tab + ((size_t)e * 32 + l) * D;
+#pragma unroll
+    for (int j = 0; j < D; j++) x[j] = p[j];
+  }
+}
+
+// Fixed-window table from slot 1 on, slot 1 = Mont(x) = t given: slots 2 .. 2^W - 1.  acc is left as the last.
+template <int TPI, int D>
+__device__ __forceinline__ void dig_fixed_table(const Group<TPI> &G, double (&acc)[D], const double (&t)[D],
+                                                const double (&n)[D], uint64_t np, uint32_t W, double *tab,
+                                                const DigSmem &sm) {
+  dig_set_b<TPI, D>(G, sm, t);
+#pragma unroll
+  for (int k = 0; k < D; k++) acc[k] = t[k];
+#pragma unroll 1
+  for (uint32_t e = 2; e < (1u << W); e++) {
+    dig_mul<TPI, D>(G, acc, acc, sm, n, np);
+    dig_slot_store<TPI, D>(tab, e, acc);
+  }
+}
+
+// acc = x^e by the fixed window over `nwin` windows of W bits from the top: W squarings and one table
+// multiply each (value 0 multiplies by Mont(1)), the entry loaded before its squarings.
+template <int TPI, int D>
+__device__ __forceinline__ void dig_fixed_scan(const Group<TPI> &G, double (&acc)[D], const ArrayView &ex, uint32_t ee,
+                                               uint32_t nwin, uint32_t W, const double (&n)[D], uint64_t np,
+                                               const double *tab, const DigSmem &sm) {
+  dig_slot_load<TPI, D>(tab, exp_window(ex, ee, (nwin - 1) * W, W), acc);
+#pragma unroll 1
+  for (int32_t wi = (int32_t)nwin - 2; wi >= 0; wi--) {
+    const uint32_t win = exp_window(ex, ee, (uint32_t)wi * W, W);
+#pragma unroll 1
+    for (uint32_t s = 0; s <= W; s++) {
+      if (s < W) {
+        dig_set_b<TPI, D>(G, sm, acc);
+      } else {
+        double y[D];
+        dig_slot_load<TPI, D>(tab, win, y);
+        dig_set_b<TPI, D>(G, sm, y);
+      }
+      dig_mul<TPI, D>(G, acc, acc, sm, n, np);
+    }
+  }
+}
+
+// As powm_instance below, on 52-bit digits.  `tab` is this warp's window table.
+template <int TPI, int L, int D, bool CT>
+__device__ __forceinline__ void dig_powm_instance(const Group<TPI> &G, const PowmArgs &args, uint32_t i, bool valid,
+                                                  double *tab, const DigSmem &sm) {
+  const uint32_t eb = in_element(args.base, i), ee = in_element(args.exp, i), em = in_element(args.mod, i);
+  const uint32_t W = args.window;
+  constexpr bool kSliding = powm_sliding(TPI, L) && !CT;
+  ExpCursor cur;
+  uint32_t nwin = 0;
+  if constexpr (kSliding) {
+    cursor_init(cur, args.exp, ee, (int32_t)exp_bitlen<TPI>(G, args.exp, ee) - 1);
+  } else if constexpr (CT) {
+    nwin = (args.exp.nlimbs * 32 + W - 1) / W;
+  } else {
+    const uint32_t ebits = __reduce_max_sync(kFull, exp_bitlen<TPI>(G, args.exp, ee));
+    nwin = ebits ? (ebits + W - 1) / W : 1;
+  }
+  double n[D], acc[D], t[D];
+  uint64_t np;
+  dig_load<TPI, D>(G, n, args.mod.limbs, args.mod.nlimbs, args.mod.stride, em);
+  {
+    uint32_t nl[L];
+    load_lane_limbs<TPI, L>(nl, args.mod.limbs, args.mod.nlimbs, args.mod.stride, em, G.lane);
+    np = dig_neg_inv(nl[0], nl[1]);
+    if (args.r2.limbs)
+      dig_load<TPI, D>(G, acc, args.r2.limbs, args.r2.nlimbs, args.r2.stride, in_element(args.r2, i));
+    else
+      dig_r2<TPI, L, D>(G, acc, nl, n, np, sm);
+  }
+  dig_set_b<TPI, D>(G, sm, acc);
+#pragma unroll
+  for (int k = 0; k < D; k++) t[k] = (G.lane == 0 && k == 0) ? 1.0 : 0.0;
+  dig_mul<TPI, D>(G, t, t, sm, n, np);  // slot 0 = Mont(1)
+  dig_slot_store<TPI, D>(tab, 0, t);
+  dig_load<TPI, D>(G, t, args.base.limbs, args.base.nlimbs, args.base.stride, eb);
+  dig_mul<TPI, D>(G, t, t, sm, n, np);  // slot 1 = Mont(x)
+  dig_slot_store<TPI, D>(tab, 1, t);
+
+  if constexpr (kSliding) {
+    // slots 2 .. 2^(W-1): Mont(x^3), Mont(x^5), ...
+    const uint32_t half = 1u << (W - 1);
+    if (half > 1) {
+      dig_set_b<TPI, D>(G, sm, t);
+      dig_mul<TPI, D>(G, acc, t, sm, n, np);  // Mont(x^2)
+      dig_set_b<TPI, D>(G, sm, acc);
+#pragma unroll 1
+      for (uint32_t j = 2; j <= half; j++) {
+        dig_mul<TPI, D>(G, t, t, sm, n, np);
+        dig_slot_store<TPI, D>(tab, j, t);
+      }
+    }
+    uint32_t sq, yidx;
+    next_window(args.exp, ee, cur, W, &sq, &yidx);
+    dig_slot_load<TPI, D>(tab, yidx, acc);
+    bool more = next_window(args.exp, ee, cur, W, &sq, &yidx);
+    uint32_t mul_at = sq;
+#pragma unroll 1
+    for (uint32_t step = 0; __any_sync(kFull, more || step < mul_at); step++) {
+      const bool use_y = step >= mul_at;
+      if (use_y) {
+        dig_slot_load<TPI, D>(tab, yidx, t);
+      } else {
+#pragma unroll
+        for (int k = 0; k < D; k++) t[k] = acc[k];
+      }
+      dig_set_b<TPI, D>(G, sm, t);
+      dig_mul<TPI, D>(G, acc, acc, sm, n, np);
+      if (use_y && more) {
+        more = next_window(args.exp, ee, cur, W, &sq, &yidx);
+        mul_at = step + 1 + sq;
+      }
+    }
+  } else {
+    dig_fixed_table<TPI, D>(G, acc, t, n, np, W, tab, sm);
+    dig_fixed_scan<TPI, D>(G, acc, args.exp, ee, nwin, W, n, np, tab, sm);
+  }
+
+  // Leave Montgomery form: acc * 1 * R^-1, then into [0, N).
+#pragma unroll
+  for (int k = 0; k < D; k++) t[k] = (G.lane == 0 && k == 0) ? 1.0 : 0.0;
+  dig_set_b<TPI, D>(G, sm, t);
+  dig_mul<TPI, D>(G, acc, acc, sm, n, np);
+  int64_t c[D];
+  dig_canon<TPI, D>(G, c, acc, n);
+  dig_store<TPI, D>(G, c, args.out, out_element(args.out, i), valid, sm);
+}
+
+// The kernels' dynamic shared memory: operand B of every warp (digits) or the four-lane squaring's blocks (limbs).
+struct PowmSmem {
+  SqrSmem sqr;
+  DigSmem dig;
+};
+template <int TPI, int L>
+__device__ __forceinline__ PowmSmem powm_smem_setup() {
+  extern __shared__ uint4 powm_dyn_smem[];
+  PowmSmem sm{};
+  if constexpr (powm_digits(TPI, L) > 0) {
+    sm.dig.b = reinterpret_cast<double *>(powm_dyn_smem) + (size_t)(threadIdx.x >> 5) * 32 * powm_digits(TPI, L);
+  } else if constexpr (powm_smem_bytes(TPI, L) > 0) {
+    sm.sqr = sqr_smem<TPI, L>(powm_dyn_smem, threadIdx.x % TPI);
+    sqr_smem_init<L>(sm.sqr);
+    __syncthreads();
+  }
+  return sm;
+}
+
 // One instance group: op instance i of `args` (every lane of the warp calls
-// this together; `valid` lanes store their result).  `slot` is this lane's
-// window-table slot (entry e at slot + e*32*L).
+// this together; `valid` lanes store their result).  `table` is this warp's
+// window table, powm_slot_words(TPI, L) words per lane and entry (limbs: this
+// lane's slot of entry e at table + lane*L + e*32*L).
 // CT (constant schedule, for secret exponents): the fixed window over the
 // exponent's whole precision for every shape -- the same sequence of
 // squarings and multiplies whatever the exponent bits, as the reference's fwe
 // scans them (powm/powm.h:39-127); the table is the fixed-window table.
 template <int TPI, int L, bool CT = false>
 __device__ __forceinline__ void powm_instance(const Group<TPI> &G, const PowmArgs &args, uint32_t i, bool valid,
-                                              uint32_t *slot, const SqrSmem &sm) {
+                                              uint32_t *table, const PowmSmem &psm) {
+  if constexpr (powm_digits(TPI, L) > 0) {
+    dig_powm_instance<TPI, L, powm_digits(TPI, L), CT>(G, args, i, valid, reinterpret_cast<double *>(table), psm.dig);
+    return;
+  } else {
+  const SqrSmem &sm = psm.sqr;
+  uint32_t *const slot = table + (size_t)(threadIdx.x & 31) * L;
   const uint32_t eb = in_element(args.base, i), ee = in_element(args.exp, i), em = in_element(args.mod, i);
 
   uint32_t n[L];
@@ -401,8 +592,20 @@ __device__ __forceinline__ void powm_instance(const Group<TPI> &G, const PowmArg
     uint32_t o = out_element(args.out, i);
     if (o < args.out.count) store_lane_limbs<TPI, L>(x, args.out.limbs, args.out.nlimbs, args.out.stride, o, G.lane);
   }
+  }
 }
 
+// Resident CTAs of 128 threads asked of the register allocator for the digit
+// kernels.  A digit product is a chain of three dependent FP64 steps, so what
+// counts is independent products in one warp, not warps: at 4 x 16 limbs (10
+// digits) 5 CTAs/SM (96 registers, spills) ran at 25.7 ms where 4 (128) take
+// 21.8 and 3 (168) 21.9; at 8 digits 6 / 5 / 4 CTAs took 33.5 / 30.4 / 29.4 ms
+// (8 x 12); at 5 digits 7 / 6 / 5 took 7.2 / 6.7 / 6.8 ms (4 x 8), with one
+// instance alone 15% faster at 5.
+constexpr int powm_min_blocks(int TPI, int L) {
+  const int D = powm_digits(TPI, L);
+  return D == 0 ? 1 : D <= 5 ? 5 : D <= 10 ? 4 : D <= 15 ? 3 : 2;
+}
 
 // Resident CTAs of 128 threads asked of the register allocator for the
 // persistent kernel: left alone, its extra loop state made the allocator take
@@ -411,38 +614,25 @@ __device__ __forceinline__ void powm_instance(const Group<TPI> &G, const PowmArg
 // choice (a bound equal to its natural count still changed its schedule and
 // cost 2.4% at 2048 bits).
 constexpr int powm_batch_min_blocks(int TPI, int L) {
+  if (powm_digits(TPI, L)) return powm_min_blocks(TPI, L);
   return (L > 8 && L <= 12) ? 5 : (TPI == 4 && L == 8) ? 4 : 1;  // 4 x 8: the squaring's state took 140
 }
 
-// The four-lane squaring's blocks (sqr.cuh) live in the kernel's dynamic shared memory.
-template <int TPI, int L>
-__device__ __forceinline__ SqrSmem powm_smem_setup() {
-  extern __shared__ uint4 powm_dyn_smem[];
-  SqrSmem sm{};
-  if constexpr (powm_smem_bytes(TPI, L) > 0) {
-    sm = sqr_smem<TPI, L>(powm_dyn_smem, threadIdx.x % TPI);
-    sqr_smem_init<L>(sm);
-    __syncthreads();
-  }
-  return sm;
-}
-
 template <int TPI, int L, bool CT = false>
-__global__ void __launch_bounds__(128) powm_kernel(PowmArgs args) {
-  const SqrSmem sm = powm_smem_setup<TPI, L>();
+__global__ void __launch_bounds__(128, powm_min_blocks(TPI, L)) powm_kernel(PowmArgs args) {
+  const PowmSmem sm = powm_smem_setup<TPI, L>();
   Group<TPI> G;
   const uint32_t gtid = blockIdx.x * blockDim.x + threadIdx.x;
   const uint32_t local = gtid / TPI;
   const bool valid = local < args.count;
   // Lanes past the end run a copy of the last instance so every shfl sees a full warp.
   const uint32_t i = args.start + (valid ? local : args.count - 1);
-  uint32_t *slot = args.table +
-                   (size_t)(gtid >> 5) * ((size_t)32 * L * powm_table_entries(args.window, powm_sliding(TPI, L) && !CT)) +
-                   (size_t)(threadIdx.x & 31) * L;
-  powm_instance<TPI, L, CT>(G, args, i, valid, slot, sm);
+  uint32_t *table = args.table + (size_t)(gtid >> 5) * ((size_t)32 * powm_slot_words(TPI, L) *
+                                                        powm_table_entries(args.window, powm_sliding(TPI, L) && !CT));
+  powm_instance<TPI, L, CT>(G, args, i, valid, table, sm);
 }
 
-// R^2 mod N (R = 2^(32 * TPI * L)) for elements start .. start+count-1 of
+// R^2 mod N (R = 2^powm_radix_bits(TPI, L)) for elements start .. start+count-1 of
 // `args.mod`, written to the same elements of `args.out` (serving set-up:
 // Montgomery constants kept on the device).
 template <int TPI, int L>
@@ -454,6 +644,17 @@ __global__ void __launch_bounds__(128) r2_kernel(PowmArgs args) {
   const uint32_t i = args.start + (valid ? local : args.count - 1);
   uint32_t n[L], r2[L];
   load_lane_limbs<TPI, L>(n, args.mod.limbs, args.mod.nlimbs, args.mod.stride, i, G.lane);
+  if constexpr (powm_digits(TPI, L) > 0) {
+    constexpr int D = powm_digits(TPI, L);
+    const DigSmem dsm = powm_smem_setup<TPI, L>().dig;
+    double nd[D], rd[D];
+    dig_load<TPI, D>(G, nd, args.mod.limbs, args.mod.nlimbs, args.mod.stride, i);
+    dig_r2<TPI, L, D>(G, rd, n, nd, dig_neg_inv(n[0], n[1]), dsm);
+    int64_t c[D];
+    dig_canon<TPI, D>(G, c, rd, nd);
+    dig_store<TPI, D>(G, c, args.out, i, valid, dsm);
+    return;
+  }
   const uint32_t np0 = neg_inv32(G.bcast(n[0], 0));
   compute_r2<TPI, L>(G, r2, n, np0);
   // the stored value must be below R and fit the output's limbs: keep it exact (< N)
@@ -481,11 +682,11 @@ struct PowmBatchArgs {
 
 template <int TPI, int L>
 __global__ void __launch_bounds__(128, powm_batch_min_blocks(TPI, L)) powm_batch_kernel(PowmBatchArgs b) {
-  const SqrSmem sm = powm_smem_setup<TPI, L>();
+  const PowmSmem sm = powm_smem_setup<TPI, L>();
   Group<TPI> G;
   const uint32_t gwarp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  uint32_t *slot = b.table + (size_t)gwarp * ((size_t)32 * L * powm_table_entries(b.window, powm_sliding(TPI, L))) +
-                   (size_t)(threadIdx.x & 31) * L;
+  uint32_t *table = b.table + (size_t)gwarp * ((size_t)32 * powm_slot_words(TPI, L) *
+                                               powm_table_entries(b.window, powm_sliding(TPI, L)));
   constexpr uint32_t per_item = 32 / TPI;
   while (true) {
     uint32_t item = 0;
@@ -500,7 +701,7 @@ __global__ void __launch_bounds__(128, powm_batch_min_blocks(TPI, L)) powm_batch
     const uint32_t i = a.start + (valid ? local : a.count - 1);
     PowmArgs args = a;
     args.window = b.window;
-    powm_instance<TPI, L>(G, args, i, valid, slot, sm);
+    powm_instance<TPI, L>(G, args, i, valid, table, sm);
   }
 }
 

@@ -108,12 +108,19 @@ struct Wave {
 };
 
 constexpr int kBuckets = 20;  // waves of 2^b .. 2^(b+1)-1 ops
+constexpr int kRadices = 4;   // Montgomery radices the kernels of one class use, at most
 
 struct Class {
   uint32_t precision = 0, n = 0, ngroups = 0, cap = 0;
   // keys
   uint32_t kcap = 0, nkeys = 0;
-  uint32_t *key_mod = nullptr, *key_r2 = nullptr;
+  uint32_t *key_mod = nullptr;
+  // R^2 mod N of every key, once per Montgomery radix of the buckets' kernels
+  uint32_t *key_r2[kRadices] = {};
+  uint32_t radix_bits[kRadices] = {};
+  int radix_bucket[kRadices] = {};  // a bucket whose kernel has that radix
+  int nradix = 0;
+  int radix[kBuckets] = {};
   std::vector<uint32_t> host_mod;  // compact rows, for the synchronous baseline
   // op slots
   uint32_t slots = 0;
@@ -215,6 +222,7 @@ static void free_all(xmpServer_t s) {
 // or the learned selector) when it runs at the class's Montgomery radix, else
 // the built-in heuristic restricted to that radix.
 static void choose_configs(xmpServer_t s, Class &c) {
+  c.nradix = 0;
   for (int b = 0; b < kBuckets; b++) {
     const uint32_t ops = 1u << b;
     PowmConfig cfg;
@@ -229,7 +237,41 @@ static void choose_configs(xmpServer_t s, Class &c) {
     // latency (one op: 3.6 vs 8.4 ms at 2048 bits, 9.2 vs 15.7 ms at 3072, 20.4 vs 30.0 ms at 4096)
     c.cta_limbs = powm_cta_limbs(c.n);
     c.cta[b] = c.cta_limbs != 0 && ops <= s->h->sm_count && powm_cta_preferred(c.n, ops, s->h->sm_count);
+    // the kernel's Montgomery radix: limb and digit kernels of one capacity differ in it
+    const uint32_t bits = powm_radix_bits(cfg.tpi, cfg.limbs);
+    int r = 0;
+    while (r < c.nradix && c.radix_bits[r] != bits) r++;
+    if (r == kRadices) {  // no room for another: the first bucket's kernel
+      c.cfg[b] = c.cfg[0];
+      c.entry[b] = c.entry[0];
+      r = c.radix[0];
+    } else if (r == c.nradix) {
+      c.radix_bits[r] = bits;
+      c.radix_bucket[r] = b;
+      c.nradix++;
+    }
+    c.radix[b] = r;
   }
+}
+
+static void one_radix(Class &c) {
+  for (int b = 1; b < kBuckets; b++) {
+    c.cfg[b] = c.cfg[0];
+    c.entry[b] = c.entry[0];
+    c.radix[b] = 0;
+  }
+  c.nradix = 1;
+}
+
+// Table words per slot: the largest any bucket's kernel needs, windows of at most `max_window` bits.
+static size_t class_table_words(Class &c, int max_window) {
+  size_t tw = 0;
+  for (int b = 0; b < kBuckets; b++) {
+    c.cfg[b].window = std::min(c.cfg[b].window, max_window);
+    tw = std::max(tw, (size_t)c.cfg[b].tpi * powm_slot_words(c.cfg[b].tpi, c.cfg[b].limbs) *
+                          powm_table_entries(c.cfg[b].window, false));
+  }
+  return tw;
 }
 
 static void fail_all(xmpServer_t s, xmpError_t e) {
@@ -295,7 +337,7 @@ static bool launch_wave(xmpServer_t s, Class &c, Wave *w, uint32_t load, uint32_
   a.base = ArrayView{c.slot_base, n, c.slots, c.slots, nullptr, 0};
   a.exp = ArrayView{c.slot_exp, n, c.slots, c.slots, nullptr, 0};
   a.mod = ArrayView{c.key_mod, n, c.kcap, c.kcap, c.slot_key, c.slots};
-  a.r2 = ArrayView{c.key_r2, n, c.kcap, c.kcap, c.slot_key, c.slots};
+  a.r2 = ArrayView{c.key_r2[c.radix[b]], n, c.kcap, c.kcap, c.slot_key, c.slots};
   a.out = OutView{c.slot_out, n, c.slots, c.slots, nullptr};
   a.start = w->first;
   a.count = w->ops;
@@ -304,7 +346,7 @@ static bool launch_wave(xmpServer_t s, Class &c, Wave *w, uint32_t load, uint32_
   if (c.cta[b] && gpu_load <= s->h->sm_count) {
     if (!powm_cta_launch(c.cta_limbs, true, a, w->ops, st)) return false;
   } else {
-    c.entry[b]->launch_ct(a, grid_for((uint64_t)w->ops * cfg.tpi, 128), st);
+    c.entry[b]->launch_ct(a, grid_for((uint64_t)w->ops * cfg.tpi, 128), 128, st);
   }
   slots_to_rows<<<dim3(div_up(w->ops, 128), c.ngroups), 128, 0, st>>>(c.slot_out, n, c.slots, w->first,
                                                                          c.rows_out + off, w->ops);
@@ -535,22 +577,32 @@ xmpError_t XMPAPI xmpServerCreate(xmpHandle_t h, const uint32_t *precisions, uin
     if (cap == 0) return fail(xmpErrorUnsupported);
     c.cap = cap;
     choose_configs(s, c);
-    size_t tw = 0;
-    for (int b = 0; b < kBuckets; b++) {
+    for (int b = 0; b < kBuckets; b++)
       if (!c.entry[b]) return fail(xmpErrorUnsupported);
-      tw = std::max(tw, (size_t)cap * powm_table_entries(c.cfg[b].window, false));
-    }
-    c.table_words = tw;
     c.kcap = round_up(cf.max_keys, 32);
-    key_bytes += 2 * (size_t)c.ngroups * 16 * c.kcap;
-    // interleaved base/exp/out + key index + compact base/exp/out + window table
-    per_slot[i] = 3 * (size_t)c.ngroups * 16 + 4 + 3 * (size_t)c.n * 4 + tw * 4;
-    per_slot_total += per_slot[i];
   }
-  if (cf.hbm_budget <= key_bytes) return fail(xmpErrorIncreaseScratchLimit);
-  // equal slot counts per class, within the budget
-  uint64_t slots = (cf.hbm_budget - key_bytes) / per_slot_total;
-  slots = std::min<uint64_t>(slots, cf.max_slots) / granule * granule;
+  // Equal slot counts per class, within the budget.  A budget too small for one granule of slots takes
+  // smaller windows, then one Montgomery radix per class (the first bucket's kernel for every wave).
+  uint64_t slots = 0;
+  for (int step = 0; step < 14 && slots < granule; step++) {
+    const int max_window = 7 - step % 7;
+    key_bytes = per_slot_total = 0;
+    for (uint32_t i = 0; i < n_classes; i++) {
+      Class &c = s->classes[i];
+      if (step == 7) {
+        choose_configs(s, c);
+        one_radix(c);
+      }
+      c.table_words = class_table_words(c, max_window);
+      key_bytes += (size_t)(1 + c.nradix) * c.ngroups * 16 * c.kcap;
+      // interleaved base/exp/out + key index + compact base/exp/out + window table
+      per_slot[i] = 3 * (size_t)c.ngroups * 16 + 4 + 3 * (size_t)c.n * 4 + c.table_words * 4;
+      per_slot_total += per_slot[i];
+    }
+    if (cf.hbm_budget <= key_bytes) continue;
+    slots = (cf.hbm_budget - key_bytes) / per_slot_total;
+    slots = std::min<uint64_t>(slots, cf.max_slots) / granule * granule;
+  }
   if (slots < granule) return fail(xmpErrorIncreaseScratchLimit);
   for (uint32_t i = 0; i < n_classes; i++) {
     Class &c = s->classes[i];
@@ -558,7 +610,8 @@ xmpError_t XMPAPI xmpServerCreate(xmpHandle_t h, const uint32_t *precisions, uin
     c.ring = SlotRing(c.slots, granule);
     const size_t gbytes = (size_t)c.ngroups * 16;
     c.key_mod = (uint32_t *)dev_alloc(s, gbytes * c.kcap);
-    c.key_r2 = (uint32_t *)dev_alloc(s, gbytes * c.kcap);
+    bool keys_ok = c.key_mod != nullptr;
+    for (int r = 0; r < c.nradix; r++) keys_ok = (c.key_r2[r] = (uint32_t *)dev_alloc(s, gbytes * c.kcap)) && keys_ok;
     c.slot_base = (uint32_t *)dev_alloc(s, gbytes * c.slots);
     c.slot_exp = (uint32_t *)dev_alloc(s, gbytes * c.slots);
     c.slot_out = (uint32_t *)dev_alloc(s, gbytes * c.slots);
@@ -567,12 +620,12 @@ xmpError_t XMPAPI xmpServerCreate(xmpHandle_t h, const uint32_t *precisions, uin
     c.rows_exp = (uint32_t *)dev_alloc(s, (size_t)c.n * 4 * c.slots);
     c.rows_out = (uint32_t *)dev_alloc(s, (size_t)c.n * 4 * c.slots);
     c.table = (uint32_t *)dev_alloc(s, c.table_words * 4 * c.slots);
-    if (!c.key_mod || !c.key_r2 || !c.slot_base || !c.slot_exp || !c.slot_out || !c.slot_key || !c.rows_base ||
+    if (!keys_ok || !c.slot_base || !c.slot_exp || !c.slot_out || !c.slot_key || !c.rows_base ||
         !c.rows_exp || !c.rows_out || !c.table)
       return fail(xmpErrorInvalidCudaMalloc);
-    if (cudaMemset(c.key_mod, 0, gbytes * c.kcap) != cudaSuccess ||
-        cudaMemset(c.key_r2, 0, gbytes * c.kcap) != cudaSuccess)
-      return fail(xmpErrorCuda);
+    if (cudaMemset(c.key_mod, 0, gbytes * c.kcap) != cudaSuccess) return fail(xmpErrorCuda);
+    for (int r = 0; r < c.nradix; r++)
+      if (cudaMemset(c.key_r2[r], 0, gbytes * c.kcap) != cudaSuccess) return fail(xmpErrorCuda);
     c.pin_base = (uint32_t *)host_alloc(s, (size_t)c.n * 4 * c.slots);
     c.pin_exp = (uint32_t *)host_alloc(s, (size_t)c.n * 4 * c.slots);
     c.pin_out = (uint32_t *)host_alloc(s, (size_t)c.n * 4 * c.slots);
@@ -643,10 +696,13 @@ xmpError_t XMPAPI xmpServerAddKeys(xmpServer_t s, uint32_t precision, const uint
                                                                                  c.n, c.kcap, c.nkeys, count);
     PowmArgs a;
     a.mod = ArrayView{c.key_mod, c.n, c.kcap, c.kcap, nullptr, 0};
-    a.out = OutView{c.key_r2, c.n, c.kcap, c.kcap, nullptr};
     a.start = c.nkeys;
     a.count = count;
-    c.entry[0]->launch_r2(a, grid_for((uint64_t)count * c.cfg[0].tpi, 128), s->setup);
+    for (int r = 0; r < c.nradix; r++) {
+      const int b = c.radix_bucket[r];
+      a.out = OutView{c.key_r2[r], c.n, c.kcap, c.kcap, nullptr};
+      c.entry[b]->launch_r2(a, grid_for((uint64_t)count * c.cfg[b].tpi, 128), 128, s->setup);
+    }
     if (cudaStreamSynchronize(s->setup) != cudaSuccess) e = xmpErrorCuda;
   }
   s->h->df(rows);

@@ -35,6 +35,7 @@
 // reduction of mont_mul would have added the products of a * a, and no block
 // is exchanged between lanes.
 #pragma once
+#include "dmont.cuh"
 #include "mont.cuh"
 
 namespace xmpb {
@@ -400,11 +401,14 @@ namespace xmpb {
 // limbs (1024 bits) +5.7%, but 4 x 12 -2% and 4 x 16 (2048 bits) -25% -- the unrolled square and
 // cross products grow with L^2 and the hot loop no longer fits the instruction cache -- so the wider
 // four-lane shapes keep mont_mul (and 4 x 16 its sliding window).
-__host__ __device__ constexpr bool powm_sqr(int TPI, int L) { return (TPI == 1 && L <= 16) || (TPI == 4 && L == 8); }
+__host__ __device__ constexpr bool powm_sqr(int TPI, int L) {
+  return !powm_digits(TPI, L) && ((TPI == 1 && L <= 16) || (TPI == 4 && L == 8));
+}
 
 // Dynamic shared memory of a 128-thread CTA of the register powm kernels.
 __host__ __device__ constexpr uint32_t powm_smem_bytes(int TPI, int L) {
-  return (TPI > 1 && powm_sqr(TPI, L)) ? sqr_smem_bytes(TPI, L) : 0u;
+  return powm_digits(TPI, L) ? 1024u * powm_digits(TPI, L)
+                             : (TPI > 1 && powm_sqr(TPI, L)) ? sqr_smem_bytes(TPI, L) : 0u;
 }
 
 // r = a^2 R^-1 mod N (almost reduced) with the shape's squaring.  r must not alias a.
