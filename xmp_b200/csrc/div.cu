@@ -17,10 +17,11 @@
 // (Moller & Granlund, "Improved division by invariant integers", IEEE TC
 // 2011, algorithm 4), refined once against the second divisor limb; the
 // multiply-subtract then needs at most one add-back.
-// Divisors above the largest register class use the same algorithm with the
-// window and divisor in the scratch arena.
+// Larger divisors (up to 512 limbs) spread divisor and window over the lanes of
+// a group; beyond that the same algorithm keeps them in the scratch arena.
 #include "internal.h"
 #include "carry.cuh"
+#include "lanes.cuh"
 #include "tune.h"
 #include <algorithm>
 
@@ -270,6 +271,141 @@ __global__ void __launch_bounds__(256) divmod_reg_kernel(DivArgs d) {
   }
 }
 
+// Divisor and window over TPI lanes x L limbs (N = TPI * L >= divisor limbs), the word above the window
+// (`top`) in every lane.  Every instance of a warp runs the quotient digits from the warp's highest down:
+// above its own highest its window is below the divisor and the digit comes out 0.  A digit: estimate from
+// the top lane's words (every lane computes it), each lane subtracts qh * V from its limbs, the lanes'
+// borrow words go one lane up, and a ballot lookahead settles what is left of them (mont.cuh).  The chain
+// from digit to digit is the bound (2048 / 1024 bits x 64 instances: 24 us against 31 us on one thread
+// each); against the scratch kernel below: 4160 / 2080 bits x 10,001 456 -> 69 us, 8192 / 4096 x 4,096
+// 1,617 -> 91 us, 16384 / 8192 x 2,048 5,533 -> 170 us.
+template <int TPI, int L>
+__global__ void __launch_bounds__(256) divmod_lanes_kernel(DivArgs d) {
+  constexpr int N = TPI * L;
+  Group<TPI> G;
+  const uint32_t local = (blockIdx.x * blockDim.x + threadIdx.x) / TPI;
+  const bool valid = local < d.count;
+  const uint32_t i = valid ? local : d.count - 1;
+  const uint32_t ea = in_element(d.a, i), eb = in_element(d.b, i);
+  const uint32_t eqo = d.q.limbs ? out_element(d.q, i) : 0, ero = d.r.limbs ? out_element(d.r, i) : 0;
+  const bool store = valid && !(d.q.limbs && eqo >= d.q.count) && !(d.r.limbs && ero >= d.r.count);
+
+  uint32_t V[L];
+  load_lane_limbs<TPI, L>(V, d.b.limbs, d.b.nlimbs, d.b.stride, eb, G.lane);
+  const uint32_t bits = dbitlen<TPI, L>(G, V);
+  const bool zero = bits == 0;  // division by zero: q = a, r = 0, written at the end
+  const int32_t bt = zero ? N - 1 : (int32_t)(bits - 1) / 32;
+  const int32_t z = N - 1 - bt;
+  const uint32_t s = zero ? 0 : (32 - bits % 32) % 32;
+  {
+    ShiftedDividend sb{&d.b, eb, z, s};
+#pragma unroll
+    for (int k = 0; k < L; k++) V[k] = sb((int32_t)(G.lane * L) + k);
+  }
+  uint32_t d1 = G.bcast(V[L - 1], TPI - 1);
+  const uint32_t d0 = G.bcast(V[L - 2], TPI - 1);
+  if (zero) d1 = 0x80000000u;
+  const uint32_t v = reciprocal_2by1(d1);
+  ShiftedCursor sa{LimbCursor{&d.a, ea, -1, make_uint4(0, 0, 0, 0)}, LimbCursor{&d.a, ea, -1, make_uint4(0, 0, 0, 0)},
+                   z, s};
+  const int32_t m = max(0, (int32_t)__reduce_max_sync(kFull, (uint32_t)max(0, (int32_t)d.a.nlimbs - bt - 1)));
+  uint32_t W[L], top = sa(m + N);
+#pragma unroll
+  for (int k = L - 1; k >= 0; k--) W[k] = sa(m + (int32_t)(G.lane * L) + k);
+
+  uint32_t qb0 = 0, qb1 = 0, qb2 = 0, qb3 = 0;
+#pragma unroll 1
+  for (int32_t j = m; j >= 0; j--) {
+    uint32_t qh = estimate_q(top, G.bcast(W[L - 1], TPI - 1), G.bcast(W[L - 2], TPI - 1), d1, d0, v, true);
+    const uint32_t next = j > 0 ? sa(j - 1) : 0u;
+    uint64_t p[L];
+    row_products<L>(p, V, qh);
+    W[0] = sub_cc(W[0], (uint32_t)p[0]);
+#pragma unroll
+    for (int k = 1; k < L; k++) W[k] = subc_cc(W[k], (uint32_t)p[k]);
+    uint32_t up = (uint32_t)(p[L - 1] >> 32) - subc(0u, 0u);
+    W[1] = sub_cc(W[1], (uint32_t)(p[0] >> 32));
+#pragma unroll
+    for (int k = 2; k < L; k++) W[k] = subc_cc(W[k], (uint32_t)(p[k - 1] >> 32));
+    up -= subc(0u, 0u);
+    // the lanes' borrow words, then the one-bit borrows that these leave
+    const uint32_t in = G.from_prev(up);
+    W[0] = sub_cc(W[0], in);
+#pragma unroll
+    for (int k = 1; k < L; k++) W[k] = subc_cc(W[k], 0u);
+    const uint32_t bo = 0u - subc(0u, 0u);
+    uint32_t any = W[0];
+#pragma unroll
+    for (int k = 1; k < L; k++) any |= W[k];
+    uint32_t out;
+    const uint32_t bin = G.lookahead(bo, any == 0u, &out);
+    W[0] = sub_cc(W[0], bin);
+#pragma unroll
+    for (int k = 1; k < L; k++) W[k] = subc_cc(W[k], 0u);
+    top -= G.bcast(up, TPI - 1) + out;
+    if (__any_sync(kFull, top != 0)) {  // an estimate was one too large: add the divisor back
+      const uint32_t msk = top != 0 ? kFull : 0u;
+      W[0] = add_cc(W[0], V[0] & msk);
+#pragma unroll
+      for (int k = 1; k < L; k++) W[k] = addc_cc(W[k], V[k] & msk);
+      const uint32_t co = addc(0u, 0u);
+      uint32_t ones = W[0];
+#pragma unroll
+      for (int k = 1; k < L; k++) ones &= W[k];
+      const uint32_t ci = G.lookahead(co, ones == kFull, &out);
+      W[0] = add_cc(W[0], ci);
+#pragma unroll
+      for (int k = 1; k < L; k++) W[k] = addc_cc(W[k], 0u);
+      qh += msk;
+    }
+    const uint32_t r4 = (uint32_t)j & 3u;
+    qb0 = r4 == 0 ? qh : qb0;
+    qb1 = r4 == 1 ? qh : qb1;
+    qb2 = r4 == 2 ? qh : qb2;
+    qb3 = r4 == 3 ? qh : qb3;
+    if (r4 == 0) {
+      const uint32_t g = (uint32_t)j >> 2;
+      if (G.lane == 0 && store && !zero && d.q.limbs && g * 4 < d.q.nlimbs)
+        store_group(d.q.limbs, d.q.nlimbs, d.q.stride, eqo, g, make_uint4(qb0, qb1, qb2, qb3));
+      qb0 = qb1 = qb2 = qb3 = 0;
+    }
+    if (j > 0) {
+      top = G.bcast(W[L - 1], TPI - 1);
+      const uint32_t below = G.lane == 0 ? next : 0u;
+      const uint32_t prev = G.from_prev(W[L - 1]);
+#pragma unroll
+      for (int k = L - 1; k > 0; k--) W[k] = W[k - 1];
+      W[0] = G.lane == 0 ? below : prev;
+    }
+  }
+  // remainder = W >> (32 z + s)
+  const uint32_t above = G.from_next(W[0]);
+  if (!store) return;
+  if (d.q.limbs) {
+    for (uint32_t g = zero ? G.lane : (uint32_t)m / 4 + 1 + G.lane; g * 4 < d.q.nlimbs; g += TPI)
+      store_group(d.q.limbs, d.q.nlimbs, d.q.stride, eqo, g,
+                  zero ? load_group(d.a.limbs, d.a.nlimbs, d.a.stride, ea, g) : make_uint4(0, 0, 0, 0));
+  }
+  if (d.r.limbs) {
+    uint32_t R[L];
+#pragma unroll
+    for (int k = 0; k < L; k++) {
+      const uint32_t hi = k + 1 < L ? W[k + 1 < L ? k + 1 : 0] : above;
+      R[k] = zero ? 0u : s ? (W[k] >> s) | (hi << (32 - s)) : W[k];
+    }
+    if (z == 0) {
+      store_lane_limbs<TPI, L>(R, d.r.limbs, d.r.nlimbs, d.r.stride, ero, G.lane);
+    } else {
+#pragma unroll
+      for (int k = 0; k < L; k++) {
+        const int32_t dst = (int32_t)(G.lane * L) + k - z;
+        if (dst >= 0) write_limb(d.r, ero, (uint32_t)dst, R[k]);
+      }
+    }
+    for (uint32_t j = N - z + G.lane; j < d.r.nlimbs; j += TPI) limb_ref(d.r.limbs, d.r.stride, ero, j) = 0;
+  }
+}
+
 // Same algorithm with the window and divisor in scratch (any divisor size).
 __global__ void __launch_bounds__(256) divmod_stream_kernel(DivArgs d) {
   uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -362,6 +498,33 @@ static DivLaunch pick_div(uint32_t nb) {
   return nullptr;
 }
 
+template <int TPI, int L>
+static void launch_div_lanes(const DivArgs &d, int threads, cudaStream_t s) {
+  divmod_lanes_kernel<TPI, L><<<grid_for((uint64_t)d.count * TPI, threads), threads, 0, s>>>(d);
+}
+// Whether lanes beat one thread per instance for a divisor that a register kernel holds: while the batch is
+// too small to give every scheduler a register warp or half of one, and the divisor long enough.  Measured,
+// register / lane kernel: 2048-bit divisors x 2^12 78.6 / 41.8 us, 2^14 78.5 / 68.8, 2^16 189 / 237; 1024 bits
+// x 2^12 31.8 / 25.6, 2^14 33.5 / 31.1, 2^16 49.7 / 70.1; 768 bits x 2^12 23.9 / 21.3, 2^14 24.7 / 25.5; 512
+// bits x 2^12 17.3 / 16.7, 2^16 23.1 / 29.1.
+static bool div_lanes_preferred(uint32_t nb, uint32_t count, uint32_t sm_count) {
+  return nb > 16 && count <= sm_count * (nb > 32 ? 128u : 64u);
+}
+
+// Lane kernel for a divisor of nb limbs (null: above 512); `wide` as in the multiply's lane path.
+static DivLaunch pick_div_lanes(uint32_t nb, uint32_t count, uint32_t sm_count) {
+  const bool wide = (uint64_t)count * round_up(nb, 16) / 16 < (uint64_t)sm_count * 4 * 2 * 32;
+  if (nb <= 16) return launch_div_lanes<2, 8>;
+  if (nb <= 32) return wide ? launch_div_lanes<4, 8> : launch_div_lanes<2, 16>;
+  if (nb <= 48) return launch_div_lanes<4, 12>;
+  if (nb <= 64) return wide ? launch_div_lanes<8, 8> : launch_div_lanes<4, 16>;
+  if (nb <= 96) return launch_div_lanes<8, 12>;
+  if (nb <= 128) return wide ? launch_div_lanes<16, 8> : launch_div_lanes<8, 16>;
+  if (nb <= 256) return wide ? launch_div_lanes<32, 8> : launch_div_lanes<16, 16>;
+  if (nb <= 512) return launch_div_lanes<32, 16>;
+  return nullptr;
+}
+
 bool div_has_register_kernel(uint32_t nb) { return pick_div(nb) != nullptr; }
 
 static xmpError_t divmod_common(xmpHandle_t h, xmpIntegers_t q, xmpIntegers_t r, xmpIntegers_t a, xmpIntegers_t b,
@@ -376,15 +539,20 @@ static xmpError_t divmod_common(xmpHandle_t h, xmpIntegers_t q, xmpIntegers_t r,
   DivLaunch launch = pol->algorithm == xmpAlgorithmDigitMP ? nullptr : pick_div(b->nlimbs);
   if (pol->algorithm == xmpAlgorithmRegMP && !launch) return xmpErrorUnsupported;
   ElemConfig cfg;
+  int source = 0;  // 1: a choice set for this very shape
   if (forced) {
     cfg = *forced;
   } else if (pol->algorithm == xmpAlgorithmDefault) {
-    int slot = tuner_lookup(h, xmpTuneDivMod, b->precision, 0, count, nullptr);
+    int slot = tuner_lookup(h, xmpTuneDivMod, b->precision, 0, count, &source);
     ElemConfig t;
     if (slot >= 0 && elem_candidate(xmpTuneDivMod, b->nlimbs, slot, &t)) cfg = t;
   }
   if (cfg.variant == 1) launch = nullptr;
   else if (!launch && forced) return xmpErrorUnsupported;
+  if ((pol->algorithm == xmpAlgorithmDefault || pol->algorithm == xmpAlgorithmDistributedMP) &&
+      (!launch || (!forced && source != 1 && div_lanes_preferred(b->nlimbs, count, h->sm_count)))) {
+    if (DivLaunch lanes = pick_div_lanes(b->nlimbs, count, h->sm_count)) launch = lanes;
+  }
   const int threads = cfg.threads;
 
   OutTarget tq, tr;

@@ -1,0 +1,45 @@
+// Integers spread over TPI lanes with L limbs each (lane g: limbs gL .. gL + L - 1): loads and stores
+// between the interleaved arrays and the lanes' registers, shared by the powm, multiply and divide kernels.
+#pragma once
+#include "internal.h"
+#include "mont.cuh"
+
+namespace xmpb {
+
+template <int TPI, int L>
+__device__ __forceinline__ void load_lane_limbs(uint32_t (&x)[L], const uint32_t *limbs, uint32_t nlimbs,
+                                                uint32_t stride, uint32_t e, uint32_t lane) {
+  const uint32_t j0 = lane * L;
+  if (L % 4 == 0) {
+#pragma unroll
+    for (int m = 0; m < L / 4; m++) {
+      uint4 v = load_group(limbs, nlimbs, stride, e, j0 / 4 + m);
+      x[4 * m] = v.x;
+      x[4 * m + 1] = v.y;
+      x[4 * m + 2] = v.z;
+      x[4 * m + 3] = v.w;
+    }
+  } else {
+#pragma unroll
+    for (int k = 0; k < L; k++) x[k] = load_limb(limbs, nlimbs, stride, e, j0 + k);
+  }
+}
+
+template <int TPI, int L>
+__device__ __forceinline__ void store_lane_limbs(const uint32_t (&x)[L], uint32_t *limbs, uint32_t nlimbs,
+                                                 uint32_t stride, uint32_t e, uint32_t lane) {
+  const uint32_t j0 = lane * L;
+  if (L % 4 == 0) {
+#pragma unroll
+    for (int m = 0; m < L / 4; m++) {
+      uint32_t g = j0 / 4 + m;
+      if (g * 4 < nlimbs) store_group(limbs, nlimbs, stride, e, g, make_uint4(x[4 * m], x[4 * m + 1], x[4 * m + 2], x[4 * m + 3]));
+    }
+  } else {
+#pragma unroll
+    for (int k = 0; k < L; k++)
+      if (j0 + k < nlimbs) limb_ref(limbs, stride, e, j0 + k) = x[k];
+  }
+}
+
+}  // namespace xmpb

@@ -13,6 +13,7 @@
 // kernels.
 #include "internal.h"
 #include "carry.cuh"
+#include "lanes.cuh"
 #include "tune.h"
 #include <algorithm>
 
@@ -116,6 +117,67 @@ __global__ void __launch_bounds__(256) mul_reg_kernel(ArrayView a, ArrayView b, 
   }
 }
 
+// Larger operand spread over TPI lanes x L limbs, one row per limb w of the smaller one: the accumulator
+// (a limb window per lane, carry words c0, c1 above it as in mont_mul) takes A * w and shifts down a word,
+// whose final product word leaves lane 0.  Rows run in steps of L (the shift is then register renaming);
+// limbs above the smaller operand read as zero.  About three instructions per limb product and no loads in
+// the rows but the smaller operand's groups, one ahead; bound by the rows' latency at small batches.
+// Measured (B200) against the streamed kernel below, which loads both limbs of every limb product: 2048 x
+// 2048 bits x 10,001 332 -> 21 us, 4096 x 4,096 1,174 -> 29 us, 8192 x 2,048 6,632 -> 52 us, 1536 x 32,768
+// 191 -> 27 us.
+template <int TPI, int L>
+__global__ void __launch_bounds__(256) mul_lanes_kernel(ArrayView a, ArrayView b, OutView c, uint32_t count) {
+  static_assert(L % 4 == 0, "whole limb groups");
+  Group<TPI> G;
+  const uint32_t local = (blockIdx.x * blockDim.x + threadIdx.x) / TPI;
+  const bool valid = local < count;
+  // lanes past the end run a copy of the last instance so every shuffle sees a full warp
+  const uint32_t i = valid ? local : count - 1;
+  const uint32_t ea = in_element(a, i), eb = in_element(b, i), ec = out_element(c, i);
+  const bool store = valid && ec < c.count;
+  uint32_t A[L], r[L], c0 = 0, c1 = 0;
+  load_lane_limbs<TPI, L>(A, a.limbs, a.nlimbs, a.stride, ea, G.lane);
+#pragma unroll
+  for (int k = 0; k < L; k++) r[k] = 0;
+  uint32_t base = 0;
+  uint4 w4 = load_group(b.limbs, b.nlimbs, b.stride, eb, 0);
+#pragma unroll 1
+  for (; base < b.nlimbs; base += L) {
+#pragma unroll
+    for (int m = 0; m < L / 4; m++) {
+      const uint32_t w[4] = {w4.x, w4.y, w4.z, w4.w};
+      w4 = load_group(b.limbs, b.nlimbs, b.stride, eb, base / 4 + m + 1);
+      uint32_t done[4];
+#pragma unroll
+      for (int t = 0; t < 4; t++) {
+        uint64_t p[L];
+        row_products<L>(p, A, w[t]);
+        add_low_halves<L>(r, c0, c1, p);
+        done[t] = r[0];
+        const uint32_t in = G.from_next(r[0]);
+        add_high_halves<L>(r, c0, c1, p);
+#pragma unroll
+        for (int j = 0; j < L - 1; j++) r[j] = r[j + 1];
+        r[L - 1] = add_cc(in, c0);
+        c0 = addc_fma(c1);
+        c1 = 0;
+      }
+      if (G.lane == 0 && store && base + 4 * m < c.nlimbs)
+        store_group(c.limbs, c.nlimbs, c.stride, ec, base / 4 + m, make_uint4(done[0], done[1], done[2], done[3]));
+    }
+  }
+  dnormalize<TPI, L>(G, r, c0);
+  if (!store) return;
+#pragma unroll
+  for (int m = 0; m < L / 4; m++) {
+    const uint32_t g = (base + G.lane * L) / 4 + m;
+    if (g * 4 < c.nlimbs)
+      store_group(c.limbs, c.nlimbs, c.stride, ec, g, make_uint4(r[4 * m], r[4 * m + 1], r[4 * m + 2], r[4 * m + 3]));
+  }
+  for (uint32_t g = (base + TPI * L) / 4 + G.lane; g * 4 < c.nlimbs; g += TPI)
+    store_group(c.limbs, c.nlimbs, c.stride, ec, g, make_uint4(0, 0, 0, 0));
+}
+
 // Column k of the product, accumulated from the interleaved arrays.
 __global__ void __launch_bounds__(256) mul_stream_kernel(ArrayView a, ArrayView b, OutView c, uint32_t count) {
   uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -157,6 +219,27 @@ static void launch_mul(ArrayView a, ArrayView b, OutView c, uint32_t count, int 
     }
   }
   mul_reg_kernel<AL, BL, false><<<grid_for(count, threads), threads, 0, s>>>(a, b, c, count);
+}
+
+template <int TPI, int L>
+static void launch_mul_lanes(ArrayView a, ArrayView b, OutView c, uint32_t count, int threads, cudaStream_t s) {
+  mul_lanes_kernel<TPI, L><<<grid_for((uint64_t)count * TPI, threads), threads, 0, s>>>(a, b, c, count);
+}
+// Lane kernel for a larger operand of n limbs (null: above 512).  12 or 16 limbs a lane; half as many over
+// twice the lanes while the batch leaves schedulers (four a SM) without a second warp.  Up to 32 limbs the
+// register kernels are faster at every batch (512 bits x 2^18: 19.8 against 28.5 us; 1024 bits 59.6 / 77.0,
+// 2^12 11.3 / 9.4), so the lanes there serve only a caller who asks for the other variant.
+static MulLaunch pick_mul_lanes(uint32_t n, uint32_t count, uint32_t sm_count) {
+  const bool wide = (uint64_t)count * round_up(n, 16) / 16 < (uint64_t)sm_count * 4 * 2 * 32;
+  if (n <= 16) return launch_mul_lanes<2, 8>;
+  if (n <= 32) return wide ? launch_mul_lanes<4, 8> : launch_mul_lanes<2, 16>;
+  if (n <= 48) return launch_mul_lanes<4, 12>;
+  if (n <= 64) return wide ? launch_mul_lanes<8, 8> : launch_mul_lanes<4, 16>;
+  if (n <= 96) return launch_mul_lanes<8, 12>;
+  if (n <= 128) return wide ? launch_mul_lanes<16, 8> : launch_mul_lanes<8, 16>;
+  if (n <= 256) return wide ? launch_mul_lanes<32, 8> : launch_mul_lanes<16, 16>;
+  if (n <= 512) return launch_mul_lanes<32, 16>;
+  return nullptr;
 }
 
 static const int kClasses[] = {2, 4, 8, 12, 16, 24, 32};
@@ -215,6 +298,7 @@ xmpError_t mul_entry(xmpHandle_t h, xmpIntegers_t p, xmpIntegers_t a, xmpInteger
   }
   if (cfg.variant == 1) launch = nullptr;
   else if (!launch && forced) return xmpErrorUnsupported;
+  if (!launch && pol->algorithm != xmpAlgorithmDigitMP) launch = pick_mul_lanes(va.nlimbs, count, h->sm_count);
   const int threads = cfg.threads;
   bool aliased = (p == a || p == b);
   bool indexed = pol->indices[0] || pol->indices[1] || pol->indices[2];

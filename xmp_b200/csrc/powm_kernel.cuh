@@ -40,7 +40,7 @@
 #pragma once
 #include "internal.h"
 #include "dmont.cuh"
-#include "mont.cuh"
+#include "lanes.cuh"
 #include "sqr.cuh"
 
 namespace xmpb {
@@ -78,42 +78,6 @@ __host__ __device__ constexpr bool powm_sliding(int TPI, int L) {
 // Fixed: slot e holds Mont(x^e), e < 2^W.
 __host__ __device__ constexpr uint32_t powm_table_entries(uint32_t W, bool sliding) {
   return sliding ? (W ? (1u << (W - 1)) + 1u : 1u) : (1u << W);
-}
-
-template <int TPI, int L>
-__device__ __forceinline__ void load_lane_limbs(uint32_t (&x)[L], const uint32_t *limbs, uint32_t nlimbs,
-                                                uint32_t stride, uint32_t e, uint32_t lane) {
-  const uint32_t j0 = lane * L;
-  if (L % 4 == 0) {
-#pragma unroll
-    for (int m = 0; m < L / 4; m++) {
-      uint4 v = load_group(limbs, nlimbs, stride, e, j0 / 4 + m);
-      x[4 * m] = v.x;
-      x[4 * m + 1] = v.y;
-      x[4 * m + 2] = v.z;
-      x[4 * m + 3] = v.w;
-    }
-  } else {
-#pragma unroll
-    for (int k = 0; k < L; k++) x[k] = load_limb(limbs, nlimbs, stride, e, j0 + k);
-  }
-}
-
-template <int TPI, int L>
-__device__ __forceinline__ void store_lane_limbs(const uint32_t (&x)[L], uint32_t *limbs, uint32_t nlimbs,
-                                                 uint32_t stride, uint32_t e, uint32_t lane) {
-  const uint32_t j0 = lane * L;
-  if (L % 4 == 0) {
-#pragma unroll
-    for (int m = 0; m < L / 4; m++) {
-      uint32_t g = j0 / 4 + m;
-      if (g * 4 < nlimbs) store_group(limbs, nlimbs, stride, e, g, make_uint4(x[4 * m], x[4 * m + 1], x[4 * m + 2], x[4 * m + 3]));
-    }
-  } else {
-#pragma unroll
-    for (int k = 0; k < L; k++)
-      if (j0 + k < nlimbs) limb_ref(limbs, stride, e, j0 + k) = x[k];
-  }
 }
 
 template <int L>
