@@ -181,7 +181,133 @@ __global__ void export_kernel(const uint32_t *__restrict__ limbs, uint32_t nlimb
   out[(size_t)dst * a.words + p] = v;
 }
 
-// Native fast paths: compact uint32 rows <-> interleaved groups, one uint4 per thread.
+// Wire rows <-> interleaved groups through a tile in shared memory, so that both sides move in whole lines:
+// the wire side in units of U (a 16-byte group, or one limb where rows or the buffer are not 16-byte
+// aligned) along the rows, the array side in groups along the instances.  Every format is a permutation
+// inside a unit and an order of units: word order reverses the units of a row and the words in a unit, byte
+// swaps stay inside a word, nails mask every word afterwards.
+// One thread per (instance, limb or word), the kernels above, reads and writes wire bytes at the rows'
+// stride: 2048-bit big-endian byte rows x 65,536 took 66 us to import and 136 to export where the tiles
+// take 9 and 8; native 256-bit rows x 2^22 to the array 61 -> 50 us, back 99 -> 45 us (16-byte pieces of
+// 32-byte rows before).
+struct WirePerm {
+  uint32_t sel;      // byte permutation of each 32-bit word of a unit
+  uint32_t flip;     // word k of a 16-byte unit comes from word k ^ flip
+  uint32_t reverse;  // units of a row in reverse order
+  uint32_t mask[2];  // nails, words of up to 64 bits
+};
+__device__ __forceinline__ uint32_t wire_unit(const WirePerm &w, uint32_t v) {
+  return __byte_perm(v, 0, w.sel) & w.mask[0];
+}
+__device__ __forceinline__ uint4 wire_unit(const WirePerm &w, uint4 v) {
+  if (w.flip & 1) v = make_uint4(v.y, v.x, v.w, v.z);
+  if (w.flip & 2) v = make_uint4(v.z, v.w, v.x, v.y);
+  return make_uint4(__byte_perm(v.x, 0, w.sel) & w.mask[0], __byte_perm(v.y, 0, w.sel) & w.mask[1],
+                    __byte_perm(v.z, 0, w.sel) & w.mask[0], __byte_perm(v.w, 0, w.sel) & w.mask[1]);
+}
+
+constexpr uint32_t kTileGroups = 32, kTileUnits = 1024;  // groups of an instance, groups in all, per tile
+
+// U: units of the wire side per group of the array side are 1 (uint4) or 4 (uint32_t).
+template <class U, bool IMPORT>
+__global__ void __launch_bounds__(256) wire_tile_kernel(U *__restrict__ wire, uint4 *__restrict__ groups,
+                                                        uint32_t units, uint32_t ngroups, uint32_t stride,
+                                                        uint32_t tile_log2, WireArgs a, WirePerm w) {
+  extern __shared__ uint4 tile[];  // [group][2^tile_log2 + 1 instances]
+  constexpr uint32_t PER = 16 / sizeof(U);
+  const uint32_t inst = 1u << tile_log2, pitch = inst + 1;
+  const uint32_t i0 = blockIdx.x << tile_log2, g0 = blockIdx.y * kTileGroups;
+  const uint32_t ng = min(kTileGroups, ngroups - g0), ni = min(inst, a.count - i0);
+  const uint32_t u0 = g0 * PER, nu = min(ng * PER, units - u0);  // this tile's units of a row
+  U *const cell = reinterpret_cast<U *>(tile);
+  if (!IMPORT) {
+    for (uint32_t e = threadIdx.x; e < ng << tile_log2; e += 256) {
+      const uint32_t g = e >> tile_log2, r = e & (inst - 1);
+      if (r < ni) tile[g * pitch + r] = __ldg(groups + (size_t)(g0 + g) * stride + i0 + r);
+    }
+    __syncthreads();
+  } else if (PER > 1) {  // limbs of the last group above the precision
+    for (uint32_t e = threadIdx.x; e < inst; e += 256) tile[(ng - 1) * pitch + e] = make_uint4(0, 0, 0, 0);
+    __syncthreads();
+  }
+  // (row, unit) of this thread's pieces, stepped without a division
+  const uint32_t dr = 256 / nu, du = 256 - dr * nu;
+  for (uint32_t r = threadIdx.x / nu, u = threadIdx.x - r * nu; r < ni; r += dr, u += du) {
+    if (u >= nu) {
+      u -= nu;
+      if (++r >= ni) break;
+    }
+    const uint32_t i = i0 + r, row = a.index ? a.index[i % a.index_count] : i;
+    const uint32_t at = w.reverse ? units - 1 - (u0 + u) : u0 + u;
+    const uint32_t c = ((u / PER) * pitch + r) * PER + u % PER;
+    if (IMPORT) {
+      U v{};
+      if (row < a.rows) v = wire_unit(w, __ldg(wire + (size_t)row * units + at));
+      cell[c] = v;
+    } else if (row < a.rows) {
+      wire[(size_t)row * units + at] = wire_unit(w, cell[c]);
+    }
+  }
+  if (IMPORT) {
+    __syncthreads();
+    for (uint32_t e = threadIdx.x; e < ng << tile_log2; e += 256) {
+      const uint32_t g = e >> tile_log2, r = e & (inst - 1);
+      if (r < ni) groups[(size_t)(g0 + g) * stride + i0 + r] = tile[g * pitch + r];
+    }
+  }
+}
+
+constexpr uint64_t kDirectBytes = 8u << 20;
+static bool wire_native(const WireArgs &a, size_t size) {
+  return size == 4 && a.order == -1 && !a.swap && a.nails == 0 && a.index == nullptr;
+}
+
+// Launches the tile kernel when the format allows it: whole 16-byte units, or single limbs for words of up
+// to four bytes.  False: the caller takes the per-word kernels.
+template <bool IMPORT>
+static bool wire_tiles(void *wire, xmpIntegers_t x, size_t size, const WireArgs &a, cudaStream_t stream) {
+  const uint64_t bytes = (uint64_t)a.words * size;
+  if (bytes != (uint64_t)x->nlimbs * 4) return false;
+  WirePerm w;
+  const bool rev = a.order == 1, swap = a.swap && size > 1;
+  w.reverse = rev;
+  w.flip = 0;
+  w.sel = 0x3210;
+  if (rev) {  // words of a unit in reverse order, then swapped inside
+    w.flip = size == 8 ? 2 : 3;
+    w.sel = size == 1 ? 0x0123 : size == 2 ? 0x1032 : 0x3210;
+  }
+  if (swap) {
+    if (size == 8) w.flip ^= 1;
+    w.sel = size == 2 ? (rev ? 0x0123 : 0x2301) : 0x0123;
+  }
+  const uint64_t m = (size == 8 ? ~0ull : (1ull << (8 * size)) - 1) >> a.nails;
+  uint64_t mm = 0;
+  for (size_t k = 0; k < 8; k += size) mm |= m << (8 * k);
+  w.mask[0] = (uint32_t)mm;
+  w.mask[1] = (uint32_t)(mm >> 32);
+  const bool vec = x->nlimbs % 4 == 0 && (uintptr_t)wire % 16 == 0;
+  if (!vec && (size == 8 || (uintptr_t)wire % 4 != 0)) return false;
+  const uint32_t ng = x->ngroups < kTileGroups ? x->ngroups : kTileGroups;
+  uint32_t lg = 5;
+  while ((ng << (lg + 1)) <= kTileUnits) lg++;
+  const dim3 grid(div_up(a.count, 1u << lg), div_up(x->ngroups, kTileGroups));
+  if (grid.y > 65535) return false;
+  const size_t smem = (size_t)ng * ((1u << lg) + 1) * 16;
+  if (vec)
+    wire_tile_kernel<uint4, IMPORT><<<grid, 256, smem, stream>>>((uint4 *)wire, (uint4 *)x->limbs, x->ngroups,
+                                                                 x->ngroups, x->stride, lg, a, w);
+  else
+    wire_tile_kernel<uint32_t, IMPORT><<<grid, 256, smem, stream>>>((uint32_t *)wire, (uint4 *)x->limbs, x->nlimbs,
+                                                                    x->ngroups, x->stride, lg, a, w);
+  return true;
+}
+
+// Native rows (compact uint32, no index) <-> interleaved groups directly, one uint4 per thread, for small
+// arrays: up to 8 MB the L2 joins the pieces of a row's sectors and a launch costs less than the tile's two
+// steps (256-bit rows x 100, three of these and an add with their copies: 59.1 us against 61.6 with tiles;
+// 2048 bits x 16,384: 7 us both ways).  Rows of a partial group come in this way at every size (1056 bits x
+// 65,536: 8.4 against 10.9 us).
 // `vec` (128-bit row access) requires nlimbs % 4 == 0 and a 16-byte aligned buffer.
 __global__ void compact_to_interleaved(const uint32_t *__restrict__ in, uint32_t *__restrict__ limbs,
                                        uint32_t nlimbs, uint32_t stride, uint32_t count, bool vec) {
@@ -519,22 +645,21 @@ static xmpError_t import_internal(xmpHandle_t handle, xmpIntegers_t out, uint32_
       return xmpErrorCuda;
     src = handle->scratch;
   }
-  bool native = (size == 4 && order == -1 && endian == native_endian() && nails == 0 && gather == nullptr);
-  if (native) {
+  WireArgs a;
+  a.words = words;
+  a.order = order;
+  a.swap = endian != native_endian();
+  a.nails = nails;
+  a.count = count;
+  a.index = gather;
+  a.index_count = policy->indices_count[0];
+  a.rows = rows;
+  if (wire_native(a, size) && (bytes <= kDirectBytes || out->nlimbs % 4 != 0)) {
     dim3 block(128), grid(grid_for(count, 128), out->ngroups);
     bool vec = (out->nlimbs % 4 == 0) && ((uintptr_t)src % 16 == 0);
     compact_to_interleaved<<<grid, block, 0, handle->stream>>>((const uint32_t *)src, out->limbs, out->nlimbs,
                                                                out->stride, count, vec);
-  } else {
-    WireArgs a;
-    a.words = words;
-    a.order = order;
-    a.swap = endian != native_endian();
-    a.nails = nails;
-    a.count = count;
-    a.index = gather;
-    a.index_count = policy->indices_count[0];
-    a.rows = rows;
+  } else if (!wire_tiles<true>(const_cast<void *>(src), out, size, a, handle->stream)) {
     uint32_t padded = round_up(out->nlimbs, 4);
     dim3 block(32, 4), grid(grid_for(count, 32), div_up(padded, 4));
     switch (size) {
@@ -585,13 +710,7 @@ static xmpError_t export_internal(xmpHandle_t handle, void *out, uint32_t *words
       if (cudaMemcpyAsync(dst, out, bytes, cudaMemcpyHostToDevice, handle->stream) != cudaSuccess) return xmpErrorCuda;
     }
   }
-  bool native = (size == 4 && order == -1 && endian == native_endian() && nails == 0 && scatter == nullptr);
-  if (native) {
-    dim3 block(128), grid(grid_for(count, 128), in->ngroups);
-    bool vec = (in->nlimbs % 4 == 0) && ((uintptr_t)dst % 16 == 0);
-    interleaved_to_compact<<<grid, block, 0, handle->stream>>>(in->limbs, in->nlimbs, in->stride, (uint32_t *)dst,
-                                                               count, vec);
-  } else if (w > 0) {
+  if (w > 0) {
     WireArgs a;
     a.words = w;
     a.order = order;
@@ -601,12 +720,19 @@ static xmpError_t export_internal(xmpHandle_t handle, void *out, uint32_t *words
     a.index = scatter;
     a.index_count = policy->indices_count[0];
     a.rows = rows;
-    dim3 block(32, 4), grid(grid_for(count, 32), div_up(w, 4));
-    switch (size) {
-      case 1: export_kernel<uint8_t><<<grid, block, 0, handle->stream>>>(in->limbs, in->nlimbs, in->stride, (uint8_t *)dst, a); break;
-      case 2: export_kernel<uint16_t><<<grid, block, 0, handle->stream>>>(in->limbs, in->nlimbs, in->stride, (uint16_t *)dst, a); break;
-      case 4: export_kernel<uint32_t><<<grid, block, 0, handle->stream>>>(in->limbs, in->nlimbs, in->stride, (uint32_t *)dst, a); break;
-      default: export_kernel<uint64_t><<<grid, block, 0, handle->stream>>>(in->limbs, in->nlimbs, in->stride, (uint64_t *)dst, a); break;
+    if (wire_native(a, size) && bytes <= kDirectBytes) {
+      dim3 block(128), grid(grid_for(count, 128), in->ngroups);
+      bool vec = (in->nlimbs % 4 == 0) && ((uintptr_t)dst % 16 == 0);
+      interleaved_to_compact<<<grid, block, 0, handle->stream>>>(in->limbs, in->nlimbs, in->stride, (uint32_t *)dst,
+                                                                 count, vec);
+    } else if (!wire_tiles<false>(dst, in, size, a, handle->stream)) {
+      dim3 block(32, 4), grid(grid_for(count, 32), div_up(w, 4));
+      switch (size) {
+        case 1: export_kernel<uint8_t><<<grid, block, 0, handle->stream>>>(in->limbs, in->nlimbs, in->stride, (uint8_t *)dst, a); break;
+        case 2: export_kernel<uint16_t><<<grid, block, 0, handle->stream>>>(in->limbs, in->nlimbs, in->stride, (uint16_t *)dst, a); break;
+        case 4: export_kernel<uint32_t><<<grid, block, 0, handle->stream>>>(in->limbs, in->nlimbs, in->stride, (uint32_t *)dst, a); break;
+        default: export_kernel<uint64_t><<<grid, block, 0, handle->stream>>>(in->limbs, in->nlimbs, in->stride, (uint64_t *)dst, a); break;
+      }
     }
   }
   if (host) {
