@@ -88,6 +88,48 @@ __device__ __forceinline__ uint32_t estimate_q(uint32_t w2, uint32_t w1, uint32_
   return qhat;
 }
 
+// Reciprocal of the normalised two-limb divisor (d1:d0) for div_3by2: floor((2^96 - 1) / (d1:d0)) - 2^32
+// (Moller & Granlund 2011, algorithm 6, from the one-limb reciprocal).
+__device__ __forceinline__ uint32_t reciprocal_3by2(uint32_t d1, uint32_t d0) {
+  uint32_t v = reciprocal_2by1(d1);
+  uint32_t p = d1 * v + d0;
+  if (p < d0) {
+    v--;
+    if (p >= d1) {
+      v--;
+      p -= d1;
+    }
+    p -= d1;
+  }
+  const uint64_t t = (uint64_t)v * d0;
+  const uint32_t t1 = (uint32_t)(t >> 32);
+  p += t1;
+  if (p < t1) {
+    v--;
+    if (((uint64_t)p << 32 | (uint32_t)t) >= ((uint64_t)d1 << 32 | d0)) v--;
+  }
+  return v;
+}
+
+// Quotient digit estimate: floor((w2:w1:w0) / (d1:d0)) for (w2:w1) <= (d1:d0), at most one too large for the
+// whole divisor (algorithm 5 of the same paper: one wide multiply by the reciprocal and two corrections
+// without branches, where a digit over d1 alone needs up to four branches to reach the same estimate).
+__device__ __forceinline__ uint32_t div_3by2(uint32_t w2, uint32_t w1, uint32_t w0, uint32_t d1, uint32_t d0,
+                                             uint32_t v) {
+  const uint64_t D = (uint64_t)d1 << 32 | d0;
+  const uint64_t u = (uint64_t)w2 << 32 | w1;
+  const uint64_t q = (uint64_t)v * w2 + u;
+  uint32_t q1 = (uint32_t)(q >> 32);
+  uint64_t r = ((uint64_t)(w1 - q1 * d1) << 32 | w0) - (uint64_t)d0 * q1 - D;
+  q1++;
+  if ((uint32_t)(r >> 32) >= (uint32_t)q) {
+    q1--;
+    r += D;
+  }
+  if (r >= D) q1++;
+  return u >= D ? 0xffffffffu : q1;
+}
+
 struct ShiftedDividend {
   const ArrayView *a;
   uint32_t e;
@@ -190,19 +232,14 @@ __global__ void __launch_bounds__(256) divmod_reg_kernel(DivArgs d) {
 #pragma unroll
     for (int k = 0; k < BN; k++) V[k] = sb(k);
   }
-  const uint32_t v = reciprocal_2by1(V[BN - 1]);
-  ShiftedCursor sa{LimbCursor{&d.a, ea, -1, make_uint4(0, 0, 0, 0)}, LimbCursor{&d.a, ea, -1, make_uint4(0, 0, 0, 0)},
-                   z, s};
   uint32_t W[BN + 1];
-#pragma unroll
-  for (int k = 0; k <= BN; k++) W[k] = sa(m + k);
-
-  // quotient limbs collect in a group buffer and are stored 128 bits at a time
-  uint32_t qb0 = 0, qb1 = 0, qb2 = 0, qb3 = 0;
-  for (int32_t j = m; j >= 0; j--) {
-    uint32_t qh = estimate_q(W[BN], W[BN - 1], BN >= 2 ? W[BN >= 2 ? BN - 2 : 0] : 0u, V[BN - 1],
-                             BN >= 2 ? V[BN >= 2 ? BN - 2 : 0] : 0u, v, BN >= 2);
-    // W -= qh * V: one mul.wide per limb; low halves at limbs 0..BN-1, high halves at 1..BN.
+  // The digit of the present window: estimate, W -= qh * V (one mul.wide per limb; low halves at limbs 0 ..
+  // BN - 1, high halves at 1 .. BN), one add-back at most.
+  const uint32_t d1 = V[BN - 1], d0 = BN >= 2 ? V[BN >= 2 ? BN - 2 : 0] : 0u;
+  const uint32_t v = BN >= 2 ? reciprocal_3by2(d1, d0) : reciprocal_2by1(d1);
+  auto digit = [&]() -> uint32_t {
+    uint32_t qh = BN >= 2 ? div_3by2(W[BN], W[BN - 1], W[BN >= 2 ? BN - 2 : 0], d1, d0, v)
+                          : estimate_q(W[BN], W[BN - 1], 0u, d1, 0u, v, false);
     uint64_t p[BN];
 #pragma unroll
     for (int k = 0; k < BN; k++) p[k] = mul_wide(qh, V[k]);
@@ -220,20 +257,80 @@ __global__ void __launch_bounds__(256) divmod_reg_kernel(DivArgs d) {
       for (int k = 1; k < BN; k++) W[k] = addc_cc(W[k], V[k]);
       W[BN] = addc(W[BN], 0u);
     }
-    const uint32_t r4 = (uint32_t)j & 3u;
-    qb0 = r4 == 0 ? qh : qb0;
-    qb1 = r4 == 1 ? qh : qb1;
-    qb2 = r4 == 2 ? qh : qb2;
-    qb3 = r4 == 3 ? qh : qb3;
-    if (r4 == 0) {
-      const uint32_t g = (uint32_t)j >> 2;
-      if (d.q.limbs && g * 4 < d.q.nlimbs) store_group(d.q.limbs, d.q.nlimbs, d.q.stride, eqo, g, make_uint4(qb0, qb1, qb2, qb3));
-      qb0 = qb1 = qb2 = qb3 = 0;
-    }
-    if (j > 0) {
+    return qh;
+  };
+  auto shift_in = [&](uint32_t limb) {
 #pragma unroll
-      for (int k = BN; k > 0; k--) W[k] = W[k - 1];
-      W[0] = sa(j - 1);
+    for (int k = BN; k > 0; k--) W[k] = W[k - 1];
+    W[0] = limb;
+  };
+  // quotient limbs collect in a group buffer and are stored 128 bits at a time
+  uint32_t qb0 = 0, qb1 = 0, qb2 = 0, qb3 = 0;
+  auto store_q = [&](uint32_t g) {
+    if (d.q.limbs && g * 4 < d.q.nlimbs)
+      store_group(d.q.limbs, d.q.nlimbs, d.q.stride, eqo, g, make_uint4(qb0, qb1, qb2, qb3));
+  };
+  if (z == 0) {
+    // A divisor of the class's length, its usual case: the dividend's limbs come group by group, the next
+    // one loaded ahead, and every digit knows its place in its group.  Against a cursor per limb (bounds, group
+    // and component tests for two limbs a digit) and the branching digit estimate, dividends twice the
+    // divisor's length: 512 bits x 262,144 63 -> 40.5 us, 1024 bits x 65,536 48 -> 30, 1536 bits x 32,768 57 ->
+    // 34.  The quotient digits' chain bounds it, 512 bits x 262,144 move at 2.9 TB/s.
+    {
+      uint32_t hi = 0;
+#pragma unroll
+      for (int k = BN; k >= 0; k--) {
+        const uint32_t lo = m + k > 0 ? load_limb(d.a.limbs, d.a.nlimbs, d.a.stride, ea, (uint32_t)(m + k - 1)) : 0u;
+        if (k < BN) W[k] = __funnelshift_l(lo, hi, s);
+        else W[k] = s ? lo >> (32 - s) : 0u;
+        hi = lo;
+      }
+    }
+    const int32_t top = (m - 1) >> 2;
+    uint4 cur = m > 0 ? load_group(d.a.limbs, d.a.nlimbs, d.a.stride, ea, (uint32_t)top) : make_uint4(0, 0, 0, 0);
+    int32_t skip = 3 - ((m - 1) & 3);  // places of the first group above the window
+#pragma unroll 1
+    for (int32_t g = top; g >= 0 && m > 0; g--) {
+      const uint4 next = g > 0 ? load_group(d.a.limbs, d.a.nlimbs, d.a.stride, ea, (uint32_t)(g - 1))
+                               : make_uint4(0, 0, 0, 0);
+      if (skip < 1) {
+        qb0 = digit();
+        store_q((uint32_t)g + 1);
+        qb1 = qb2 = qb3 = 0;
+        shift_in(__funnelshift_l(cur.z, cur.w, s));
+      }
+      if (skip < 2) {
+        qb3 = digit();
+        shift_in(__funnelshift_l(cur.y, cur.z, s));
+      }
+      if (skip < 3) {
+        qb2 = digit();
+        shift_in(__funnelshift_l(cur.x, cur.y, s));
+      }
+      qb1 = digit();
+      shift_in(__funnelshift_l(next.w, cur.x, s));
+      cur = next;
+      skip = 0;
+    }
+    qb0 = digit();
+    store_q(0);
+  } else {
+    ShiftedCursor sa{LimbCursor{&d.a, ea, -1, make_uint4(0, 0, 0, 0)},
+                     LimbCursor{&d.a, ea, -1, make_uint4(0, 0, 0, 0)}, z, s};
+#pragma unroll
+    for (int k = 0; k <= BN; k++) W[k] = sa(m + k);
+    for (int32_t j = m; j >= 0; j--) {
+      const uint32_t qh = digit();
+      const uint32_t r4 = (uint32_t)j & 3u;
+      qb0 = r4 == 0 ? qh : qb0;
+      qb1 = r4 == 1 ? qh : qb1;
+      qb2 = r4 == 2 ? qh : qb2;
+      qb3 = r4 == 3 ? qh : qb3;
+      if (r4 == 0) {
+        store_q((uint32_t)j >> 2);
+        qb0 = qb1 = qb2 = qb3 = 0;
+      }
+      if (j > 0) shift_in(sa(j - 1));
     }
   }
   // limbs above the quotient's top group
@@ -305,7 +402,7 @@ __global__ void __launch_bounds__(256) divmod_lanes_kernel(DivArgs d) {
   uint32_t d1 = G.bcast(V[L - 1], TPI - 1);
   const uint32_t d0 = G.bcast(V[L - 2], TPI - 1);
   if (zero) d1 = 0x80000000u;
-  const uint32_t v = reciprocal_2by1(d1);
+  const uint32_t v = reciprocal_3by2(d1, d0);
   ShiftedCursor sa{LimbCursor{&d.a, ea, -1, make_uint4(0, 0, 0, 0)}, LimbCursor{&d.a, ea, -1, make_uint4(0, 0, 0, 0)},
                    z, s};
   const int32_t m = max(0, (int32_t)__reduce_max_sync(kFull, (uint32_t)max(0, (int32_t)d.a.nlimbs - bt - 1)));
@@ -316,7 +413,7 @@ __global__ void __launch_bounds__(256) divmod_lanes_kernel(DivArgs d) {
   uint32_t qb0 = 0, qb1 = 0, qb2 = 0, qb3 = 0;
 #pragma unroll 1
   for (int32_t j = m; j >= 0; j--) {
-    uint32_t qh = estimate_q(top, G.bcast(W[L - 1], TPI - 1), G.bcast(W[L - 2], TPI - 1), d1, d0, v, true);
+    uint32_t qh = div_3by2(top, G.bcast(W[L - 1], TPI - 1), G.bcast(W[L - 2], TPI - 1), d1, d0, v);
     const uint32_t next = j > 0 ? sa(j - 1) : 0u;
     uint64_t p[L];
     row_products<L>(p, V, qh);
