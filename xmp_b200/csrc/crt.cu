@@ -21,37 +21,38 @@ std::vector<CrtKernelEntry> &crt_registry() {
   }                                                                                               \
   static CrtKernelRegistrar crt_reg_##TPI##_##L(TPI, L, crt_launch_##TPI##_##L);
 
-// Shapes for halves of 256 to 4096 bits (RSA-512 to RSA-8192): two per size.
+// Shapes for halves of 256 to 4096 bits (RSA-512 to RSA-8192): two or more per size, from the fewest lanes
+// (digit kernels: most throughput) to the shortest latency.
 XMPB_REGISTER_CRT(4, 2)
 XMPB_REGISTER_CRT(8, 1)
+XMPB_REGISTER_CRT(1, 16)
 XMPB_REGISTER_CRT(4, 4)
 XMPB_REGISTER_CRT(8, 2)
+XMPB_REGISTER_CRT(1, 24)
 XMPB_REGISTER_CRT(4, 6)
 XMPB_REGISTER_CRT(8, 3)
+XMPB_REGISTER_CRT(1, 32)
+XMPB_REGISTER_CRT(2, 16)
 XMPB_REGISTER_CRT(4, 8)
 XMPB_REGISTER_CRT(8, 4)
+XMPB_REGISTER_CRT(2, 24)
 XMPB_REGISTER_CRT(4, 12)
 XMPB_REGISTER_CRT(8, 6)
 XMPB_REGISTER_CRT(4, 16)
 XMPB_REGISTER_CRT(8, 8)
+XMPB_REGISTER_CRT(4, 24)
 XMPB_REGISTER_CRT(8, 12)
 XMPB_REGISTER_CRT(16, 6)
 XMPB_REGISTER_CRT(8, 16)
 XMPB_REGISTER_CRT(16, 8)
 
+// The shape with the lowest expected time for the batch (two lane groups an instance).
 CrtConfig crt_config(uint32_t nlimbs, uint32_t exp_bits, uint32_t count, uint32_t sm_count) {
   CrtConfig best;
   double best_score = 1e300;
-  const double want_threads = (double)sm_count * 4 * 32;
   for (const auto &e : crt_registry()) {
-    const uint32_t cap = (uint32_t)(e.tpi * e.limbs);
-    if (cap < nlimbs) continue;
-    // the powm heuristic's cost model: padding squared, lane overhead, starved SMs below 4 warps each
-    const double pad = (double)cap / nlimbs;
-    const double work = pad * pad * (4.0 * e.limbs + 12.0) / (4.0 * e.limbs);
-    const double threads = (double)count * e.tpi * 2;  // a pair of groups per instance
-    const double starve = threads < want_threads ? want_threads / threads : 1.0;
-    const double score = work * starve;
+    if ((uint32_t)(e.tpi * e.limbs) < nlimbs) continue;
+    const double score = powm_shape_cycles(e.tpi, e.limbs, 2.0 * count, sm_count);
     if (score < best_score) {
       best_score = score;
       best.tpi = e.tpi;

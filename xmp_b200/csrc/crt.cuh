@@ -116,8 +116,7 @@ __device__ __forceinline__ void crt_reduce(const Group<TPI> &G, uint32_t (&xm)[L
 template <int TPI, int L>
 __device__ __forceinline__ void powm_fixed_full(const Group<TPI> &G, uint32_t (&acc)[L], const uint32_t (&xm)[L],
                                                 const ArrayView &ex, uint32_t ee, uint32_t nbits,
-                                                const uint32_t (&n)[L], uint32_t np0, uint32_t W, uint32_t *slot,
-                                                const SqrSmem &sm) {
+                                                const uint32_t (&n)[L], uint32_t np0, uint32_t W, uint32_t *slot) {
   const size_t es = (size_t)32 * L;
   uint32_t t[L], y[L];
 #pragma unroll
@@ -143,7 +142,7 @@ __device__ __forceinline__ void powm_fixed_full(const Group<TPI> &G, uint32_t (&
     win = exp_window(ex, ee, (uint32_t)wi * W, W);
 #pragma unroll 1
     for (uint32_t s = 0; s < W; s++) {
-      mont_square<TPI, L>(G, t, acc, n, np0, sm);
+      mont_square<TPI, L>(G, t, acc, n, np0);
 #pragma unroll
       for (int k = 0; k < L; k++) acc[k] = t[k];
     }
@@ -339,7 +338,7 @@ __device__ __forceinline__ void dig_crt_instance(const Group<TPI> &G, const CrtA
   dig_slot_store<TPI, D>(tab, 1, t);
   const uint32_t ee = in_element(ev, i);
   dig_fixed_table<TPI, D>(G, acc, t, n, np, W, tab, sm);
-  dig_fixed_scan<TPI, D>(G, acc, ev, ee, nwin, W, n, np, tab, sm);
+  dig_fixed_scan<TPI, L, D, false>(G, acc, ev, ee, nwin, W, n, np, tab, sm);
 #pragma unroll
   for (int k = 0; k < D; k++) t[k] = (G.lane == 0 && k == 0) ? 1.0 : 0.0;
   dig_set_b<TPI, D>(G, sm, t);
@@ -392,7 +391,7 @@ __host__ __device__ constexpr uint32_t crt_table_entries(int TPI, int L, uint32_
 template <int TPI, int L>
 __global__ void __launch_bounds__(128, powm_min_blocks(TPI, L)) crt_kernel(CrtArgs a) {
   static_assert(TPI <= 16, "both groups of a pair sit in one warp");
-  const PowmSmem psm = powm_smem_setup<TPI, L>();
+  const DigSmem sm = powm_smem_setup<TPI, L>();
   Group<TPI> G;
   const uint32_t gtid = blockIdx.x * blockDim.x + threadIdx.x;
   const uint32_t local = gtid / (2 * TPI);
@@ -403,10 +402,9 @@ __global__ void __launch_bounds__(128, powm_min_blocks(TPI, L)) crt_kernel(CrtAr
   uint32_t *table = a.table + (size_t)(gtid >> 5) * ((size_t)32 * powm_slot_words(TPI, L) *
                                                      crt_table_entries(TPI, L, a.window));
   if constexpr (powm_digits(TPI, L) > 0) {
-    dig_crt_instance<TPI, L, powm_digits(TPI, L)>(G, a, i, valid, second, reinterpret_cast<double *>(table), psm.dig);
+    dig_crt_instance<TPI, L, powm_digits(TPI, L)>(G, a, i, valid, second, reinterpret_cast<double *>(table), sm);
     return;
   } else {
-  const SqrSmem &sm = psm.sqr;
   uint32_t *const slot = table + (size_t)(threadIdx.x & 31) * L;
   const ArrayView mv = second ? a.q : a.p, ov = second ? a.p : a.q, ev = second ? a.dq : a.dp;
   const uint32_t em = in_element(mv, i);
@@ -426,7 +424,7 @@ __global__ void __launch_bounds__(128, powm_min_blocks(TPI, L)) crt_kernel(CrtAr
   uint32_t one[L], acc[L], mine[L], other[L];
 #pragma unroll
   for (int k = 0; k < L; k++) one[k] = (G.lane == 0 && k == 0) ? 1u : 0u;
-  powm_fixed_full<TPI, L>(G, acc, xm, ev, in_element(ev, i), nbits, n, np0, a.window, slot, sm);
+  powm_fixed_full<TPI, L>(G, acc, xm, ev, in_element(ev, i), nbits, n, np0, a.window, slot);
   mont_mul<TPI, L>(G, mine, acc, one, n, np0);
   dreduce<TPI, L>(G, mine, n);
 #pragma unroll

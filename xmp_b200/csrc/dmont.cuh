@@ -113,6 +113,14 @@ __device__ __forceinline__ void dig_settle(const Group<TPI> &G, double (&r)[D], 
   for (int j = 0; j < D; j++) r[j] = __dadd_rn(r[j], __hiloint2double(0x43300000, (int)(j ? up[j ? j - 1 : 0] : in)));
 }
 
+// Rows a step of dig_mul unrolls; the exponentiation loop's code must fit the instruction cache: all of
+// them up to ten digits without the square (4 x 16, ten rows: 21.6 ms; five 21.6 and a lone instance 3.2
+// instead of 3.0 ms), five with it (1 x 16 4.92 / 4.88 ms; 1 x 32 22.7 / 21.5) and at fifteen digits (4 x 24
+// 54.0 / 46.7 ms), two at twenty (2 x 32: 57.1 ms with all, 42.1 with five, 40.5).
+__host__ __device__ constexpr int dig_mul_step(int TPI, int D) {
+  return D == 20 && TPI > 1 ? 2 : D == 15 || D == 20 || (TPI == 1 && D == 10) ? 5 : D;
+}
+
 // r = a * B * R^-1 mod N (|r| <= N), B the operand in shared memory.  n: the
 // modulus's digits; np = -N^-1 mod 2^52 (lane 0's is used).  r may alias a.
 // A row adds a * b_i and n * q with q fixing column 0 mod 2^52, and drops that
@@ -121,10 +129,11 @@ __device__ __forceinline__ void dig_settle(const Group<TPI> &G, double (&r)[D], 
 // the order of the additions is free: a * b_(i+1) is added between the
 // quotient digit and the products that wait for it, which hides the digit's
 // latency (a lone 1024-bit chain on 4 lanes: 3.25 -> 2.15 us a product).
+// The shift is register renaming inside a step of U rows and D + 2 register moves from step to step.
 template <int TPI, int D>
 __device__ __forceinline__ void dig_mul(const Group<TPI> &G, double (&r)[D], const double (&a)[D], const DigSmem &sm,
                                         const double (&n)[D], uint64_t np) {
-  constexpr int N = TPI * D, STEP = 32 / TPI;
+  constexpr int N = TPI * D, STEP = 32 / TPI, U = dig_mul_step(TPI, D);
   const double *bp = dig_b<TPI, D>(sm);
   uint64_t col[D + 2];
 #pragma unroll
@@ -133,14 +142,14 @@ __device__ __forceinline__ void dig_mul(const Group<TPI> &G, double (&r)[D], con
   const uint32_t lane0 = G.lane == 0 ? kFull : 0u;
   dig_row<D, 0>(col, a, bp[0]);
 #pragma unroll 1
-  for (int src = 0; src < TPI; src++) {
+  for (int i = 0; i < N; i += U) {
 #pragma unroll
-    for (int row = 0; row < D; row++) {
+    for (int row = 0; row < U; row++) {
       const uint64_t x = col[0] * np;
       double q = __dsub_rn(__hiloint2double((int)(((uint32_t)(x >> 32) & 0xfffffu) ^ 0x43380000u), (int)(uint32_t)x),
                            0x1.8p52);  // low 52 bits, balanced
       q = dig_bcast<TPI>(q, 0);
-      if (row + 1 < D || src + 1 < TPI) dig_row<D, 1>(col, a, bp[(src * D + row + 1) * STEP]);
+      if (row + 1 < U || i + U < N) dig_row<D, 1>(col, a, bp[(i + row + 1) * STEP]);
       dig_row<D, 0>(col, n, q);
       int32_t c = (int32_t)((uint32_t)(col[0] >> 32) - k) >> 20;
       k += (2u * kDigLoBits + kDigHiPairBits) << 20;
@@ -162,6 +171,82 @@ __device__ __forceinline__ void dig_mul(const Group<TPI> &G, double (&r)[D], con
   const uint32_t p0 = G.lane * D;
   dig_settle<TPI, D>(G, r, col, (2u * (N - 1 - p0) * kDigLoBits + (N - p0) * kDigHiPairBits) << 20,
                      (2u * kDigLoBits + kDigHiPairBits) << 20);
+}
+
+// ---- squares, one lane an instance ----------------------------------------------------
+//
+// r = a^2 R^-1: the square's 2D columns first, each digit product a_i a_j (i < j) once and doubled, then the
+// reduction's rows n * q alone on them: D (D + 1) / 2 + D^2 digit products instead of 2 D^2.  Columns start
+// from minus the constant of the halves they will take, so the reduction's constants are its own.
+constexpr uint64_t kDigLoBits64 = (uint64_t)kDigLoBits << 52, kDigHiBits64 = (0x467ull << 52) + (1ull << 51);
+// Digit pairs (i, j), i < j < D, with i + j = c.
+__host__ __device__ constexpr int dig_cross_pairs(int c, int D) {
+  const int lo = c - D + 1 > 0 ? c - D + 1 : 0, end = (c + 1) / 2;
+  return c < 0 || end < lo ? 0 : end - lo;
+}
+// Half the constant of column c of a square of D digits formed as twice its cross products plus its squares.
+__host__ __device__ constexpr uint64_t dig_square_const(int c, int D) {
+  return (uint64_t)dig_cross_pairs(c, D) * kDigLoBits64 + (uint64_t)dig_cross_pairs(c - 1, D) * kDigHiBits64 +
+         (c % 2 ? kDigHiBits64 : kDigLoBits64) / 2;
+}
+
+// s = the 2D columns of a^2, as true signed sums.
+template <int D>
+__device__ __forceinline__ void dig_block_square(uint64_t (&s)[2 * D], const double (&a)[D]) {
+#pragma unroll
+  for (int c = 0; c < 2 * D; c++) s[c] = 0 - dig_square_const(c, D);
+#pragma unroll
+  for (int i = 0; i + 1 < D; i++) {
+    double h[D], t[D];
+#pragma unroll
+    for (int j = i + 1; j < D; j++) h[j] = __fma_rz(a[i], a[j], kDigHi);
+#pragma unroll
+    for (int j = i + 1; j < D; j++) t[j] = __dsub_rn(kDigLo, h[j]);
+#pragma unroll
+    for (int j = i + 1; j < D; j++) t[j] = __fma_rz(a[i], a[j], t[j]);
+#pragma unroll
+    for (int j = i + 1; j < D; j++) {
+      s[i + j] += dig_bits(t[j]);
+      s[i + j + 1] += dig_bits(h[j]);
+    }
+  }
+  double h[D], t[D];
+#pragma unroll
+  for (int j = 0; j < D; j++) h[j] = __fma_rz(a[j], a[j], kDigHi);
+#pragma unroll
+  for (int j = 0; j < D; j++) t[j] = __dsub_rn(kDigLo, h[j]);
+#pragma unroll
+  for (int j = 0; j < D; j++) t[j] = __fma_rz(a[j], a[j], t[j]);
+#pragma unroll
+  for (int j = 0; j < D; j++) {
+    s[2 * j] = 2 * s[2 * j] + dig_bits(t[j]);
+    s[2 * j + 1] = 2 * s[2 * j + 1] + dig_bits(h[j]);
+  }
+}
+
+// r = a^2 R^-1 mod N (|r| <= N).  r may alias a.  A row makes column 0 of what is left 0 mod 2^52 and drops it;
+// k is the high word of the constant that the halves of n * q have left in it (the low word stays 0).
+template <int D>
+__device__ __forceinline__ void dig_sqr1(const Group<1> &G, double (&r)[D], const double (&a)[D], const double (&n)[D],
+                                         uint64_t np) {
+  uint64_t col[2 * D];
+  dig_block_square<D>(col, a);
+  uint32_t k = 0;
+  constexpr uint32_t kstep = (uint32_t)((kDigLoBits64 + kDigHiBits64) >> 32);
+#pragma unroll
+  for (int row = 0; row < D; row++) {
+    const uint64_t x = (((uint64_t)((uint32_t)(col[0] >> 32) - k) << 32) | (uint32_t)col[0]) * np;
+    const double q = __dsub_rn(
+        __hiloint2double((int)(((uint32_t)(x >> 32) & 0xfffffu) ^ 0x43380000u), (int)(uint32_t)x), 0x1.8p52);
+    dig_row<D, 0>(col, n, q);
+    const int32_t c = (int32_t)((uint32_t)(col[0] >> 32) - k - (kDigLoBits << 20)) >> 20;
+    k += kstep;
+#pragma unroll
+    for (int j = 0; j < 2 * D - 1; j++) col[j] = col[j + 1];
+    col[0] += (uint64_t)(int64_t)c;
+  }
+  // column p collected D - 1 - p low and D - p high halves of n * q
+  dig_settle<1, D>(G, r, col, (uint32_t)(((D - 1) * kDigLoBits64 + D * kDigHiBits64) >> 32), kstep);
 }
 
 // ---- limbs <-> digits ----------------------------------------------------------------
@@ -318,9 +403,9 @@ __device__ __forceinline__ void dig_r2(const Group<TPI> &G, double (&r2)[D], con
 // digits are faster throughout (2048 bits, 4 x 16: 36.6 / 21.8 ms, one instance 4.73 / 3.03 ms; 4 x 8:
 // 10.3 / 6.7 ms; 8 x 12: 42.9 / 29.4 ms; 1 x 8: 1.13 / 0.85 ms; 16 x 6, 22.5 / 17.9 ms, is the least),
 // below that the few digits hold too much padding (4 x 4: three digits a lane for 128 bits, 1.0x at the
-// full batch and 0.76x at a sixteenth; 16 x 3: 1.18x and 0.88x; 8 x 5: 0.9x; 1 x 7: 1.03x and 0.9x).
+// full batch and 0.76x at a sixteenth; 16 x 3: 1.18x and 0.88x; 8 x 5: 0.9x; 1 x 5: 0.95x).
 __host__ __device__ constexpr int powm_digits(int TPI, int L) {
-  return L >= 6 && L != 7 ? dig_count(TPI, L) : 0;
+  return L >= 6 ? dig_count(TPI, L) : 0;
 }
 
 // Words per lane of one window-table entry.
@@ -332,5 +417,14 @@ __host__ __device__ constexpr int powm_slot_words(int TPI, int L) {
 __host__ __device__ constexpr uint32_t powm_radix_bits(int TPI, int L) {
   return powm_digits(TPI, L) ? 52u * TPI * powm_digits(TPI, L) : 32u * TPI * L;
 }
+
+// Whether the digit kernel squares with dig_sqr1.  Measured against the same kernels squaring with dig_mul:
+// 256 bits 0.85 -> 0.77 ms (151,552 instances, 512-bit exponents), 512 bits 5.6 -> 4.9, 768 bits 13.3 ->
+// 11.4, 1024 bits 28 -> 21.5; one 512-bit instance 0.77 -> 0.66 ms.  Over two and four
+// lanes the same saving (each lane its block's square, the block pairs shared out, columns through the
+// thread's shared memory) measured no faster at a full batch and slower below (2 x 16: 1.73x against 1.71x of
+// the limb kernel's rate at the full batch, 1.29x against 1.58x for one instance; 4 x 16: 1.64x / 1.68x and
+// 1.27x / 1.56x): without a * b's products in the rows nothing hides the quotient digits' latency.
+__host__ __device__ constexpr bool powm_dig_sqr(int TPI, int L) { return powm_digits(TPI, L) > 0 && TPI == 1; }
 
 }  // namespace xmpb

@@ -99,6 +99,15 @@ PowmConfig powm_default_config(uint32_t nlimbs, uint32_t exp_bits, uint32_t coun
                                uint32_t sm_count, uint32_t cap = 0);
 bool powm_config_valid(const PowmConfig &c, uint32_t nlimbs);
 
+// Scheduler cycles of one Montgomery product on the register kernel of a shape: of one instance alone, and
+// what an instance adds to a scheduler's load when the GPU is full.
+struct PowmShapeCost {
+  double latency, work;
+};
+PowmShapeCost powm_shape_cost(int tpi, int limbs);
+// Expected cycles of a product step of `groups` lane groups on an otherwise idle GPU.
+double powm_shape_cycles(int tpi, int limbs, double groups, uint32_t sm_count);
+
 // Runs out = base^exp mod mod for `count` op instances starting at 0 with the
 // given configuration (validation already done).  Chunks the launch so the
 // window tables fit the scratch limit.

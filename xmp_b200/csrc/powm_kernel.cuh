@@ -61,14 +61,14 @@ struct PowmArgs {
 // sweep of every registered kernel with both methods (a batch that fills the
 // GPU, fractions of it and a single instance).  The sliding window does ~3-4%
 // fewer Montgomery multiplies but adds per-step control.  Digit kernels: it
-// wins except on one lane and on two lanes up to 8 limbs, where the instances
-// of a warp read their table entries from as many places and the control is a
-// larger share (2048 bits, 4 x 16: 21.8 against 22.4 ms; 256 bits, 1 x 8: 1.01
-// against 0.85 ms; 2 x 8: 3.73 against 3.58).  Limb kernels (below six limbs a
+// wins except on one lane (which squares with dig_sqr1, on steps all instances
+// of the warp share) and on two lanes up to 8 limbs, where the control is a
+// larger share (2048 bits, 4 x 16: 21.8 against 22.4 ms; 2 x 8: 3.73 against
+// 3.58).  Limb kernels (below six limbs a
 // lane): where it was faster at the batch and the batch and single-instance
 // gains together were positive (1280 bits, 8 x 5: +8.1%; 16 x 4: +3.3%).
 __host__ __device__ constexpr bool powm_sliding(int TPI, int L) {
-  return powm_digits(TPI, L) ? TPI >= 4 || (TPI == 2 && L >= 12) || L >= 24
+  return powm_digits(TPI, L) ? TPI >= 4 || (TPI == 2 && L >= 12)
                              : (TPI == 4 && L == 5) || (TPI == 8 && (L == 4 || L == 5)) ||
                                    (TPI == 16 && (L == 2 || L == 4));
 }
@@ -205,6 +205,27 @@ __device__ __forceinline__ uint32_t exp_bitlen(const Group<TPI> &G, const ArrayV
 
 // ---- exponentiation on 52-bit digits (dmont.cuh) ------------------------------------
 
+// Exponents with few one bits (public ones: 65537) need no window table: the window for this warp, W or 1,
+// whichever takes fewer multiplies.  `bits` is the longest exponent of the warp.  Sliding windows: each
+// instance multiplies at its own ones.  Fixed windows multiply where any instance has a one, which is only
+// looked at for short exponents (up to 256 bits).  2048-bit moduli, e = 65537 x 50,001: 1.62 -> 1.40 ms.
+template <int TPI, bool SLIDING>
+__device__ __forceinline__ uint32_t dig_window(const Group<TPI> &G, const ArrayView &ex, uint32_t e, uint32_t bits,
+                                               uint32_t W) {
+  uint32_t ones = 0;
+  if constexpr (SLIDING) {
+    for (uint32_t j = G.lane; j < ex.nlimbs; j += TPI) ones += __popc(load_limb(ex.limbs, ex.nlimbs, ex.stride, e, j));
+#pragma unroll
+    for (int o = TPI / 2; o > 0; o >>= 1) ones += __shfl_xor_sync(kFull, ones, o, TPI);
+    ones = __reduce_max_sync(kFull, ones);
+    return ones <= (1u << (W - 1)) + bits / (W + 1) ? 1u : W;
+  }
+  if (ex.nlimbs > 8) return W;
+  for (uint32_t j = 0; j < ex.nlimbs; j++)
+    ones += __popc(__reduce_or_sync(kFull, load_limb(ex.limbs, ex.nlimbs, ex.stride, e, j)));
+  return ones <= (1u << W) - 2 + (bits + W - 1) / W ? 1u : W;
+}
+
 // Window table of one warp: entry e of this lane's digits.  From four lanes an instance on, digit j of the
 // 32 lanes lies together (the lanes of an instance read whole 32-byte sectors); below that a lane's digits do.
 template <int TPI, int D>
@@ -262,8 +283,9 @@ __device__ __forceinline__ void dig_fixed_table(const Group<TPI> &G, double (&ac
 }
 
 // acc = x^e by the fixed window over `nwin` windows of W bits from the top: W squarings and one table
-// multiply each (value 0 multiplies by Mont(1)), the entry loaded before its squarings.
-template <int TPI, int D>
+// multiply each.  SKIP (public exponents): no multiply where every instance of the warp has a zero window;
+// otherwise value 0 multiplies by Mont(1).
+template <int TPI, int L, int D, bool SKIP>
 __device__ __forceinline__ void dig_fixed_scan(const Group<TPI> &G, double (&acc)[D], const ArrayView &ex, uint32_t ee,
                                                uint32_t nwin, uint32_t W, const double (&n)[D], uint64_t np,
                                                const double *tab, const DigSmem &sm) {
@@ -271,16 +293,30 @@ __device__ __forceinline__ void dig_fixed_scan(const Group<TPI> &G, double (&acc
 #pragma unroll 1
   for (int32_t wi = (int32_t)nwin - 2; wi >= 0; wi--) {
     const uint32_t win = exp_window(ex, ee, (uint32_t)wi * W, W);
+    const bool mul = !SKIP || __any_sync(kFull, win != 0);
+    if constexpr (powm_dig_sqr(TPI, L)) {
 #pragma unroll 1
-    for (uint32_t s = 0; s <= W; s++) {
-      if (s < W) {
-        dig_set_b<TPI, D>(G, sm, acc);
-      } else {
+      for (uint32_t s = 0; s < W; s++) {
+        dig_sqr1<D>(G, acc, acc, n, np);
+      }
+      if (mul) {
         double y[D];
         dig_slot_load<TPI, D>(tab, win, y);
         dig_set_b<TPI, D>(G, sm, y);
+        dig_mul<TPI, D>(G, acc, acc, sm, n, np);
       }
-      dig_mul<TPI, D>(G, acc, acc, sm, n, np);
+    } else {
+#pragma unroll 1
+      for (uint32_t s = 0; s < W + (mul ? 1u : 0u); s++) {
+        if (s < W) {
+          dig_set_b<TPI, D>(G, sm, acc);
+        } else {
+          double y[D];
+          dig_slot_load<TPI, D>(tab, win, y);
+          dig_set_b<TPI, D>(G, sm, y);
+        }
+        dig_mul<TPI, D>(G, acc, acc, sm, n, np);
+      }
     }
   }
 }
@@ -290,17 +326,18 @@ template <int TPI, int L, int D, bool CT>
 __device__ __forceinline__ void dig_powm_instance(const Group<TPI> &G, const PowmArgs &args, uint32_t i, bool valid,
                                                   double *tab, const DigSmem &sm) {
   const uint32_t eb = in_element(args.base, i), ee = in_element(args.exp, i), em = in_element(args.mod, i);
-  const uint32_t W = args.window;
+  uint32_t W = args.window;
   constexpr bool kSliding = powm_sliding(TPI, L) && !CT;
   ExpCursor cur;
   uint32_t nwin = 0;
-  if constexpr (kSliding) {
-    cursor_init(cur, args.exp, ee, (int32_t)exp_bitlen<TPI>(G, args.exp, ee) - 1);
-  } else if constexpr (CT) {
+  if constexpr (CT) {
     nwin = (args.exp.nlimbs * 32 + W - 1) / W;
   } else {
-    const uint32_t ebits = __reduce_max_sync(kFull, exp_bitlen<TPI>(G, args.exp, ee));
-    nwin = ebits ? (ebits + W - 1) / W : 1;
+    const uint32_t mine = exp_bitlen<TPI>(G, args.exp, ee);
+    const uint32_t ebits = __reduce_max_sync(kFull, mine);
+    W = dig_window<TPI, kSliding>(G, args.exp, ee, ebits, W);
+    if constexpr (kSliding) cursor_init(cur, args.exp, ee, (int32_t)mine - 1);
+    else nwin = ebits ? (ebits + W - 1) / W : 1;
   }
   double n[D], acc[D], t[D];
   uint64_t np;
@@ -359,7 +396,7 @@ __device__ __forceinline__ void dig_powm_instance(const Group<TPI> &G, const Pow
     }
   } else {
     dig_fixed_table<TPI, D>(G, acc, t, n, np, W, tab, sm);
-    dig_fixed_scan<TPI, D>(G, acc, args.exp, ee, nwin, W, n, np, tab, sm);
+    dig_fixed_scan<TPI, L, D, !CT>(G, acc, args.exp, ee, nwin, W, n, np, tab, sm);
   }
 
   // Leave Montgomery form: acc * 1 * R^-1, then into [0, N).
@@ -372,23 +409,11 @@ __device__ __forceinline__ void dig_powm_instance(const Group<TPI> &G, const Pow
   dig_store<TPI, D>(G, c, args.out, out_element(args.out, i), valid, sm);
 }
 
-// The kernels' dynamic shared memory: operand B of every warp (digits) or the four-lane squaring's blocks (limbs).
-struct PowmSmem {
-  SqrSmem sqr;
-  DigSmem dig;
-};
+// This warp's operand B in the kernel's dynamic shared memory (digit kernels).
 template <int TPI, int L>
-__device__ __forceinline__ PowmSmem powm_smem_setup() {
+__device__ __forceinline__ DigSmem powm_smem_setup() {
   extern __shared__ uint4 powm_dyn_smem[];
-  PowmSmem sm{};
-  if constexpr (powm_digits(TPI, L) > 0) {
-    sm.dig.b = reinterpret_cast<double *>(powm_dyn_smem) + (size_t)(threadIdx.x >> 5) * 32 * powm_digits(TPI, L);
-  } else if constexpr (powm_smem_bytes(TPI, L) > 0) {
-    sm.sqr = sqr_smem<TPI, L>(powm_dyn_smem, threadIdx.x % TPI);
-    sqr_smem_init<L>(sm.sqr);
-    __syncthreads();
-  }
-  return sm;
+  return DigSmem{reinterpret_cast<double *>(powm_dyn_smem) + (size_t)(threadIdx.x >> 5) * 32 * powm_digits(TPI, L)};
 }
 
 // One instance group: op instance i of `args` (every lane of the warp calls
@@ -401,12 +426,11 @@ __device__ __forceinline__ PowmSmem powm_smem_setup() {
 // scans them (powm/powm.h:39-127); the table is the fixed-window table.
 template <int TPI, int L, bool CT = false>
 __device__ __forceinline__ void powm_instance(const Group<TPI> &G, const PowmArgs &args, uint32_t i, bool valid,
-                                              uint32_t *table, const PowmSmem &psm) {
+                                              uint32_t *table, const DigSmem &sm) {
   if constexpr (powm_digits(TPI, L) > 0) {
-    dig_powm_instance<TPI, L, powm_digits(TPI, L), CT>(G, args, i, valid, reinterpret_cast<double *>(table), psm.dig);
+    dig_powm_instance<TPI, L, powm_digits(TPI, L), CT>(G, args, i, valid, reinterpret_cast<double *>(table), sm);
     return;
   } else {
-  const SqrSmem &sm = psm.sqr;
   uint32_t *const slot = table + (size_t)(threadIdx.x & 31) * L;
   const uint32_t eb = in_element(args.base, i), ee = in_element(args.exp, i), em = in_element(args.mod, i);
 
@@ -521,7 +545,7 @@ __device__ __forceinline__ void powm_instance(const Group<TPI> &G, const PowmArg
       if constexpr (powm_sqr(TPI, L)) {
 #pragma unroll 1
         for (uint32_t s = 0; s < W; s++) {
-          mont_square<TPI, L>(G, x, acc, n, np0, sm);
+          mont_square<TPI, L>(G, x, acc, n, np0);
 #pragma unroll
           for (int k = 0; k < L; k++) acc[k] = x[k];
         }
@@ -565,10 +589,11 @@ __device__ __forceinline__ void powm_instance(const Group<TPI> &G, const PowmArg
 // digits) 5 CTAs/SM (96 registers, spills) ran at 25.7 ms where 4 (128) take
 // 21.8 and 3 (168) 21.9; at 8 digits 6 / 5 / 4 CTAs took 33.5 / 30.4 / 29.4 ms
 // (8 x 12); at 5 digits 7 / 6 / 5 took 7.2 / 6.7 / 6.8 ms (4 x 8), with one
-// instance alone 15% faster at 5.
+// instance alone 15% faster at 5; at 15 digits 3 / 2 took 46.7 / 44.9 ms
+// (4 x 24) and 13.2 / 11.4 ms (1 x 24, with the square's 30 columns).
 constexpr int powm_min_blocks(int TPI, int L) {
   const int D = powm_digits(TPI, L);
-  return D == 0 ? 1 : D <= 5 ? 5 : D <= 10 ? 4 : D <= 15 ? 3 : 2;
+  return D == 0 ? 1 : D <= 5 ? 5 : D <= 10 ? 4 : 2;
 }
 
 // Resident CTAs of 128 threads asked of the register allocator for the
@@ -579,12 +604,12 @@ constexpr int powm_min_blocks(int TPI, int L) {
 // cost 2.4% at 2048 bits).
 constexpr int powm_batch_min_blocks(int TPI, int L) {
   if (powm_digits(TPI, L)) return powm_min_blocks(TPI, L);
-  return (L > 8 && L <= 12) ? 5 : (TPI == 4 && L == 8) ? 4 : 1;  // 4 x 8: the squaring's state took 140
+  return 1;
 }
 
 template <int TPI, int L, bool CT = false>
 __global__ void __launch_bounds__(128, powm_min_blocks(TPI, L)) powm_kernel(PowmArgs args) {
-  const PowmSmem sm = powm_smem_setup<TPI, L>();
+  const DigSmem sm = powm_smem_setup<TPI, L>();
   Group<TPI> G;
   const uint32_t gtid = blockIdx.x * blockDim.x + threadIdx.x;
   const uint32_t local = gtid / TPI;
@@ -610,7 +635,7 @@ __global__ void __launch_bounds__(128) r2_kernel(PowmArgs args) {
   load_lane_limbs<TPI, L>(n, args.mod.limbs, args.mod.nlimbs, args.mod.stride, i, G.lane);
   if constexpr (powm_digits(TPI, L) > 0) {
     constexpr int D = powm_digits(TPI, L);
-    const DigSmem dsm = powm_smem_setup<TPI, L>().dig;
+    const DigSmem dsm = powm_smem_setup<TPI, L>();
     double nd[D], rd[D];
     dig_load<TPI, D>(G, nd, args.mod.limbs, args.mod.nlimbs, args.mod.stride, i);
     dig_r2<TPI, L, D>(G, rd, n, nd, dig_neg_inv(n[0], n[1]), dsm);
@@ -646,7 +671,7 @@ struct PowmBatchArgs {
 
 template <int TPI, int L>
 __global__ void __launch_bounds__(128, powm_batch_min_blocks(TPI, L)) powm_batch_kernel(PowmBatchArgs b) {
-  const PowmSmem sm = powm_smem_setup<TPI, L>();
+  const DigSmem sm = powm_smem_setup<TPI, L>();
   Group<TPI> G;
   const uint32_t gwarp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   uint32_t *table = b.table + (size_t)gwarp * ((size_t)32 * powm_slot_words(TPI, L) *

@@ -8,4 +8,6 @@ XMPB_REGISTER_POWM(2, 6)
 XMPB_REGISTER_POWM(2, 8)
 XMPB_REGISTER_POWM(2, 12)
 XMPB_REGISTER_POWM(2, 16)
+XMPB_REGISTER_POWM(2, 24)
+XMPB_REGISTER_POWM(2, 32)
 }  // namespace xmpb

@@ -11,4 +11,6 @@ XMPB_REGISTER_POWM(4, 8)
 XMPB_REGISTER_POWM(4, 10)
 XMPB_REGISTER_POWM(4, 12)
 XMPB_REGISTER_POWM(4, 16)
+XMPB_REGISTER_POWM(4, 24)
+XMPB_REGISTER_POWM(4, 32)
 }  // namespace xmpb

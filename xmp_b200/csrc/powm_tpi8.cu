@@ -11,4 +11,5 @@ XMPB_REGISTER_POWM(8, 8)
 XMPB_REGISTER_POWM(8, 10)
 XMPB_REGISTER_POWM(8, 12)
 XMPB_REGISTER_POWM(8, 16)
+XMPB_REGISTER_POWM(8, 24)
 }  // namespace xmpb

@@ -12,28 +12,6 @@
 //
 // Per-thread (TPI = 1): T is formed in registers; the reduction takes T's low
 // half as the accumulator and shifts T's high words in at the top.
-//
-// Four lanes (TPI = 4, lane g holding block A_g of L limbs): every lane
-// computes the same three products, each with a partner lane chosen by its
-// own index, so the lanes run one instruction stream and the work is even:
-//   S = A_g^2 (lane-local, doubled cross products plus the squares of the
-//       limbs), at word offset 2gL of T;
-//   P = 2 A_g A_h, h = g + 1 mod 4 (the partner's words arrive by shuffle), at
-//       offset L(g + h): the adjacent block pairs (0,1) (1,2) (2,3) (3,0);
-//   Q = half of 2 A_g A_h, h = g + 2 mod 4: the pairs (0,2) and (1,3) are
-//       split between their two lanes -- lanes 0, 1 take their own low half
-//       against all of the partner's words, lanes 2, 3 all of their own words
-//       against the partner's high half (two passes of L/2 x L/2) -- at offset
-//       L(g + h) (+ L/2 for lanes 2, 3).
-// Together these are every block pair (g, h), g <= h, once, cross pairs
-// doubled.  Each product is cut into L-word blocks kept in this thread's
-// shared memory.  A block at T offset o belongs in lane g's accumulator window
-// when the reduction reaches row o - gL; every such row is a multiple of L/2,
-// so at each half-block boundary every lane adds the (at most two) blocks the
-// schedule gives it -- the same instructions in every lane, a shared zero
-// block where a lane has none.  The words of T thus enter exactly where the
-// reduction of mont_mul would have added the products of a * a, and no block
-// is exchanged between lanes.
 #pragma once
 #include "dmont.cuh"
 #include "mont.cuh"
@@ -112,19 +90,15 @@ __device__ __forceinline__ void mont_sqr1(const Group<1> &G, uint32_t (&r)[L], c
   dsub<1, L>(G, r, n, 0u - c0);
 }
 
-// ---- several lanes -----------------------------------------------------------------
+// ---- several lanes: the schedule of an even split -------------------------------------
 //
-// T lanes (T = 2, 4), lane g holding block A_g of L limbs.  Every lane
-// computes, in one instruction stream, its own square S, the products
-// P_r = 2 A_g A_{g+r mod T} for r = 1 .. T/2 - 1, and Q, the half of
-// 2 A_g A_{g+T/2 mod T} that falls to it (lanes g < T/2 take their own low half
-// against all of the partner's words, lanes g >= T/2 all of their own words
-// against the partner's high half).  Block ids per lane: 0 S lo, 1 S hi,
-// 2r and 2r + 1 the low and high blocks of P_r, T and T + 1 those of Q.
-// The offsets and boundaries below are defined for any even T; the lane plan
-// (two 4-bit block ids at each of the 2T + 1 boundaries, 24 nibbles) holds
-// T <= 4.  Eight lanes would need a wider plan and measured no faster (8 x 4
-// limbs at 1024 bits: 21% slower than mont_mul), so they are not offered.
+// T lanes (T = 2, 4), lane g holding block A_g of L words.  Every lane computes, in one instruction stream,
+// its own square S, the products P_r = 2 A_g A_{g+r mod T} for r = 1 .. T/2 - 1, and Q, the half of
+// 2 A_g A_{g+T/2 mod T} that falls to it (lanes g < T/2 take their own low half against all of the partner's
+// words, lanes g >= T/2 all of their own words against the partner's high half).  Block ids per lane: 0 S lo,
+// 1 S hi, 2r and 2r + 1 the low and high blocks of P_r, T and T + 1 those of Q.  The functions say where each
+// block belongs; no kernel squares over several lanes at present (limbs: 4 x 8 was 5.7% faster than a general
+// product and gave way to the digit kernels; digits: see powm_dig_sqr).
 
 // T-word offset of block `id` of lane g (T lanes, L limbs each).
 __host__ __device__ constexpr int sqr_block_offset(int T, int L, int g, int id) {
@@ -189,236 +163,20 @@ __host__ __device__ constexpr uint64_t sqr_slots_mask(int T) {
   return mask;
 }
 
-// This thread's blocks in the kernel's dynamic shared memory.  Block b, group m
-// (4 words) of thread t is blocks[(b * L/4 + m) * 128 + t]: a warp moves 512
-// contiguous bytes per access.  extra[(r - 1) * 128 + t] holds the word of P_r
-// above its high block; zero is one all-zero block shared by the CTA.
-struct SqrSmem {
-  uint4 *blocks;
-  uint32_t *extra;
-  const uint4 *zero;
-  uint32_t tid;
-  SqrPlanBits plan;
-};
+// Limb kernels whose exponentiation squares with the specialised product: one lane, up to five limbs (more take
+// the digit kernels, which have a square of their own).  They use the fixed window (every instance of a warp
+// squares at the same steps; the sliding window is not combined with it).
+__host__ __device__ constexpr bool powm_sqr(int TPI, int L) { return !powm_digits(TPI, L) && TPI == 1; }
 
-// Dynamic shared memory of a 128-thread CTA of the T-lane squaring kernels.
-__host__ __device__ constexpr uint32_t sqr_smem_bytes(int T, int L) {
-  return (uint32_t)((T + 2) * L * 128 * 4 + L * 4 + (T / 2 > 1 ? T / 2 - 1 : 1) * 128 * 4);
-}
-
-template <int T, int L>
-__device__ __forceinline__ SqrSmem sqr_smem(uint4 *base, uint32_t lane) {
-  SqrSmem s;
-  s.blocks = base;
-  s.zero = base + (T + 2) * (L / 4) * 128;
-  s.extra = reinterpret_cast<uint32_t *>(base + (T + 2) * (L / 4) * 128 + L / 4);
-  s.tid = threadIdx.x;
-  s.plan = sqr_lane_plan<T>(lane);
-  return s;
-}
-
-// Zeroes the shared zero block; every thread of the CTA calls it before a __syncthreads.
-template <int L>
-__device__ __forceinline__ void sqr_smem_init(const SqrSmem &s) {
-  if (s.tid < (uint32_t)(L / 4)) const_cast<uint4 *>(s.zero)[s.tid] = make_uint4(0, 0, 0, 0);
-}
-
-// Stores words [OFF, OFF + L) of x as block b.
-template <int L, int OFF, int N>
-__device__ __forceinline__ void sqr_store(const SqrSmem &s, int b, const uint32_t (&x)[N]) {
-#pragma unroll
-  for (int m = 0; m < L / 4; m++) {
-    uint4 v;
-    v.x = OFF + 4 * m + 0 < N ? x[OFF + 4 * m + 0 < N ? OFF + 4 * m + 0 : 0] : 0u;
-    v.y = OFF + 4 * m + 1 < N ? x[OFF + 4 * m + 1 < N ? OFF + 4 * m + 1 : 0] : 0u;
-    v.z = OFF + 4 * m + 2 < N ? x[OFF + 4 * m + 2 < N ? OFF + 4 * m + 2 : 0] : 0u;
-    v.w = OFF + 4 * m + 3 < N ? x[OFF + 4 * m + 3 < N ? OFF + 4 * m + 3 : 0] : 0u;
-    s.blocks[(b * (L / 4) + m) * 128 + s.tid] = v;
-  }
-}
-
-// Adds this lane's block in slot `slot` of boundary b (none: the zero block) into the window.
-template <int T, int L>
-__device__ __forceinline__ void sqr_add(const SqrSmem &s, uint32_t b, uint32_t slot, uint32_t (&r)[L], uint32_t &c0,
-                                        uint32_t &c1) {
-  const uint32_t nib = 2 * b + slot;
-  const uint32_t word = nib < 8 ? s.plan.w[0] : (nib < 16 ? s.plan.w[1] : s.plan.w[2]);
-  const uint32_t id = (word >> (4 * (nib % 8))) & 15u;
-  const bool has = id < (uint32_t)(T + 2);
-  const uint4 *p = has ? s.blocks + (size_t)id * (L / 4) * 128 + s.tid : s.zero;
-  const uint32_t step = has ? 128u : 1u;
-  uint32_t v[L];
-#pragma unroll
-  for (int m = 0; m < L / 4; m++) {
-    uint4 g = p[m * step];
-    v[4 * m] = g.x;
-    v[4 * m + 1] = g.y;
-    v[4 * m + 2] = g.z;
-    v[4 * m + 3] = g.w;
-  }
-  // the high block of P_r (odd id below T) carries one more word, at the lane's carry word
-  const bool extra = has && id >= 2 && id < (uint32_t)T && (id & 1u);
-  const uint32_t e = extra ? s.extra[(id / 2 - 1) * 128 + s.tid] : 0u;
-  r[0] = add_cc(r[0], v[0]);
-#pragma unroll
-  for (int k = 1; k < L; k++) r[k] = addc_cc(r[k], v[k]);
-  c0 = addc_cc(c0, e);
-  c1 = addc(c1, 0u);
-}
-
-// x (H + 1 words) = 2 * a[lo, lo + H) as a number of its own.
-template <int L, int H>
-__device__ __forceinline__ void sqr_double_half(uint32_t (&x)[H + 1], const uint32_t (&a)[L], int lo) {
-  x[0] = a[lo] << 1;
-#pragma unroll
-  for (int j = 1; j < H; j++) x[j] = __funnelshift_l(a[lo + j - 1], a[lo + j], 1);
-  x[H] = a[lo + H - 1] >> 31;
-}
-
-// r = a^2 R^-1 mod N (almost reduced) over T lanes.  r must not alias a.
-template <int T, int L>
-__device__ __forceinline__ void mont_sqr_lanes(const Group<T> &G, uint32_t (&r)[L], const uint32_t (&a)[L],
-                                               const uint32_t (&n)[L], uint32_t np0, const SqrSmem &sm) {
-  static_assert(L % 4 == 0 && (T == 2 || T == 4), "lane squaring: T in {2, 4}, L a multiple of 4");
-  constexpr int H = L / 2;
-  // S = A_g^2
-  {
-    uint32_t s[2 * L];
-    lane_square<L>(s, a);
-    sqr_store<L, 0>(sm, 0, s);
-    sqr_store<L, L>(sm, 1, s);
-  }
-  // P_r = 2 A_g A_h, h = g + r mod T
-  if constexpr (T > 2) {
-    uint32_t d[L + 1];
-    d[0] = a[0] << 1;
-#pragma unroll
-    for (int j = 1; j < L; j++) d[j] = __funnelshift_l(a[j - 1], a[j], 1);
-    d[L] = a[L - 1] >> 31;
-#pragma unroll
-    for (int rr = 1; rr < T / 2; rr++) {
-      const uint32_t h = (G.lane + rr) % T;
-      uint32_t R[2 * L + 1];
-#pragma unroll
-      for (int k = 0; k < 2 * L + 1; k++) R[k] = 0;
-#pragma unroll
-      for (int k = 0; k < L; k++) {
-        const uint32_t w = G.bcast(a[k], h);
-        uint64_t p[L];
-#pragma unroll
-        for (int j = 0; j < L; j++) p[j] = mul_wide(d[j], w);
-        const uint32_t top = d[L] ? w : 0u;
-        R[k] = add_cc(R[k], (uint32_t)p[0]);
-#pragma unroll
-        for (int j = 1; j < L; j++) R[k + j] = addc_cc(R[k + j], (uint32_t)p[j]);
-        R[k + L] = addc_cc(R[k + L], top);
-        R[k + L + 1] = addc(R[k + L + 1], 0u);
-        R[k + 1] = add_cc(R[k + 1], (uint32_t)(p[0] >> 32));
-#pragma unroll
-        for (int j = 1; j < L; j++) R[k + 1 + j] = addc_cc(R[k + 1 + j], (uint32_t)(p[j] >> 32));
-        R[k + L + 1] = addc(R[k + L + 1], 0u);
-      }
-      sqr_store<L, 0>(sm, 2 * rr, R);
-      sqr_store<L, L>(sm, 2 * rr + 1, R);
-      sm.extra[(rr - 1) * 128 + sm.tid] = R[2 * L];
-    }
-  }
-  // Q: the half of 2 A_g A_h, h = g + T/2 mod T, that falls to this lane
-  {
-    const uint32_t h = (G.lane + T / 2) % T;
-    const bool first = G.lane < (uint32_t)(T / 2);
-    uint32_t dl[H + 1], dh[H + 1];
-    sqr_double_half<L, H>(dl, a, 0);
-    sqr_double_half<L, H>(dh, a, H);
-    uint32_t Q[L + H + 1];
-#pragma unroll
-    for (int k = 0; k < L + H + 1; k++) Q[k] = 0;
-#pragma unroll
-    for (int pass = 0; pass < 2; pass++) {
-      uint32_t x[H + 1];
-#pragma unroll
-      for (int j = 0; j <= H; j++) x[j] = (pass == 0 || first) ? dl[j] : dh[j];
-#pragma unroll
-      for (int k = 0; k < H; k++) {
-        // each lane sends the word its receiver needs: a first lane (the receiver of a second one) takes
-        // word pass*H + k, a second lane (the receiver of a first one) word H + k
-        const uint32_t send = first ? a[H + k] : a[pass * H + k];
-        const uint32_t w = G.bcast(send, h);
-        uint64_t p[H];
-#pragma unroll
-        for (int j = 0; j < H; j++) p[j] = mul_wide(x[j], w);
-        const uint32_t top = x[H] ? w : 0u;
-        const int o = pass * H + k;
-        Q[o] = add_cc(Q[o], (uint32_t)p[0]);
-#pragma unroll
-        for (int j = 1; j < H; j++) Q[o + j] = addc_cc(Q[o + j], (uint32_t)p[j]);
-        Q[o + H] = addc_cc(Q[o + H], top);
-        Q[o + H + 1] = addc(Q[o + H + 1], 0u);
-        Q[o + 1] = add_cc(Q[o + 1], (uint32_t)(p[0] >> 32));
-#pragma unroll
-        for (int j = 1; j < H; j++) Q[o + 1 + j] = addc_cc(Q[o + 1 + j], (uint32_t)(p[j] >> 32));
-        Q[o + H + 1] = addc(Q[o + H + 1], 0u);
-      }
-    }
-    sqr_store<L, 0>(sm, T, Q);
-    sqr_store<L, L>(sm, T + 1, Q);  // words L .. L + H of Q, zeros above
-  }
-  // reduction, the blocks of T entering at the half-block boundaries
-  uint32_t c0 = 0, c1 = 0;
-#pragma unroll
-  for (int k = 0; k < L; k++) r[k] = 0;
-  sqr_add<T, L>(sm, 0, 0, r, c0, c1);
-#pragma unroll 1
-  for (int src = 0; src < T; src++) {
-#pragma unroll
-    for (int k = 0; k < L; k++) {
-      if (k == 0 || k == H) {
-        const uint32_t b = 2 * src + (k == H ? 1 : 0);
-        if (b > 0) {
-          // blocks at this boundary: the same count for every lane (warp-uniform)
-          constexpr uint64_t kSlots = sqr_slots_mask(T);
-          const uint32_t slots = (uint32_t)(kSlots >> (2 * b)) & 3u;
-          if (slots > 0) sqr_add<T, L>(sm, b, 0, r, c0, c1);
-          if (slots > 1) sqr_add<T, L>(sm, b, 1, r, c0, c1);
-        }
-      }
-      redc_row<T, L>(G, r, c0, c1, n, np0, 0u);
-    }
-  }
-  sqr_add<T, L>(sm, 2 * T, 0, r, c0, c1);
-  const uint32_t ovf = dnormalize<T, L>(G, r, c0);
-  dsub<T, L>(G, r, n, 0u - ovf);
-}
-
-}  // namespace xmpb
-
-namespace xmpb {
-
-// Register kernels whose exponentiation squares with the specialised product.  They use the fixed
-// window (every instance of a warp squares at the same steps; the sliding window is not combined with
-// it).  Measured on B200 against the same kernels squaring with mont_mul (CUDA events, full waves, every
-// result checked): per-thread 16 limbs (512 bits) +12.5%, 8 limbs (256 bits) +16%; four lanes x 8
-// limbs (1024 bits) +5.7%, but 4 x 12 -2% and 4 x 16 (2048 bits) -25% -- the unrolled square and
-// cross products grow with L^2 and the hot loop no longer fits the instruction cache -- so the wider
-// four-lane shapes keep mont_mul (and 4 x 16 its sliding window).
-__host__ __device__ constexpr bool powm_sqr(int TPI, int L) {
-  return !powm_digits(TPI, L) && ((TPI == 1 && L <= 16) || (TPI == 4 && L == 8));
-}
-
-// Dynamic shared memory of a 128-thread CTA of the register powm kernels.
-__host__ __device__ constexpr uint32_t powm_smem_bytes(int TPI, int L) {
-  return powm_digits(TPI, L) ? 1024u * powm_digits(TPI, L)
-                             : (TPI > 1 && powm_sqr(TPI, L)) ? sqr_smem_bytes(TPI, L) : 0u;
-}
+// Dynamic shared memory of a 128-thread CTA of the register powm kernels: the digit kernels' operand B.
+__host__ __device__ constexpr uint32_t powm_smem_bytes(int TPI, int L) { return 1024u * powm_digits(TPI, L); }
 
 // r = a^2 R^-1 mod N (almost reduced) with the shape's squaring.  r must not alias a.
 template <int TPI, int L>
 __device__ __forceinline__ void mont_square(const Group<TPI> &G, uint32_t (&r)[L], const uint32_t (&a)[L],
-                                            const uint32_t (&n)[L], uint32_t np0, const SqrSmem &sm) {
-  if constexpr (TPI == 1 && powm_sqr(TPI, L)) {
+                                            const uint32_t (&n)[L], uint32_t np0) {
+  if constexpr (powm_sqr(TPI, L)) {
     mont_sqr1<L>(G, r, a, n, np0);
-  } else if constexpr (TPI > 1 && powm_sqr(TPI, L)) {
-    mont_sqr_lanes<TPI, L>(G, r, a, n, np0, sm);
   } else {
     mont_mul<TPI, L>(G, r, a, a, n, np0);
   }
