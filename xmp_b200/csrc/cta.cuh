@@ -1,444 +1,287 @@
 // Latency distribution: one exponentiation per CTA.
 //
-// The lane kernels (powm_kernel.cuh) multiply by interleaved CIOS, whose n
-// rows per Montgomery product each wait on the previous row's quotient digit:
-// a lone 2048-bit exponentiation on one warp (32 lanes x 2 limbs) takes 8 ms,
-// the floor under a server's latency.  Here a CTA of (n/4)^2 threads forms a
-// Montgomery product as three whole-operand products with no digit-serial
-// dependency (separated operand scanning, Montgomery's REDC on the whole low
-// half):
-//   T = a b,   m = (T mod R) N' mod R   (N' = -N^-1 mod R),   U = T + m N,
-//   r = U / R  (< 2N; one conditional subtraction of N makes it < N).
-// Each product x y (n words each) is cut into 4 x 4-word tiles, one per thread
-// (16 mul.wide; four row chains added as a tree give the tile's exact 8-word
-// product); the tiles on one anti-diagonal share a word offset, so thread
-// (d, w) sums word w of the tiles of diagonal d (64-bit accumulators, no
-// carries yet) into a word-linear array (low and high tile halves apart);
-// one warp then resolves n words, K = n/32 per lane: each word's column sum,
-// the bits above 32 of the two words below folded in, and the remaining
-// one-bit carries by a ballot lookahead (the incoming carries of 32 lanes are
-// the bits of (P + 2G + cin) xor P).  Of U only the high half is resolved and
-// of T only the low half (the product schedule below).  A product costs 3
-// barriers, a Montgomery product 9.  Operands, the window table and all
-// intermediates live in the CTA's shared memory.  It does not reach the lane
+// The lane kernels (powm_kernel.cuh) multiply row by row, each row waiting on
+// the previous one's quotient digit: a lone 2048-bit exponentiation takes 8 ms
+// on them, the floor under a server's latency.  Here a CTA forms a Montgomery
+// product as three whole-operand products with no digit-serial dependency
+// (Montgomery's REDC on the whole low half):
+//   T = a b,   m = (T mod R) N' mod R   (N' = -N^-1 mod R),   U = T + m N,   r = U / R,
+// on balanced 52-bit digits in doubles with columns that do not carry
+// (dmont.cuh).  P lanes share the columns c and N + c of a product, which
+// together have a term for every digit of x: lane p multiplies x_i by
+// y_((c - i) mod N), i = p mod P (y is stored twice, so that no index wraps), and
+// adds the halves to its sums of one column or the other.  Shuffles add the
+// lanes' sums, each step halving the sums that a lane holds; a column is its low
+// halves and the high halves of the column below, and one step of carries, each
+// column's to the next, makes digits of them.  No resolution is needed because
+// operands need not be canonical:
+//   - m is only needed mod R, so the carry out of its top digit is dropped;
+//   - T's upper columns stay in the lanes' sums, to which m N's are added;
+//   - U's low half is a multiple c R of R, so c is read off its two top
+//     columns, whatever is below them being far less than half of R.
+// Values stay within |v| <= N: |ab| / R + N / 2 since R >= 4 N.  A product is
+// three times [terms, barrier, digits, barrier], 300 instructions a warp at 40
+// digits, and takes 2,100 cycles: the scheduler issues in 35% of them, the rest
+// waits on the chain of FP64 steps, shuffles and barriers.  P sets the length of
+// that chain: 2048 bits take 3.53 / 2.56 / 2.95 ms with 4 / 8 / 16 lanes, 4096
+// bits 12.8 / 9.75 ms with 4 / 8, 1024 bits 0.99 / 1.01 ms with 4 / 8.  Against
+// 4 x 4-word tiles of 32-bit words summed through shared memory and resolved by
+// a single warp's ballot lookahead (9 barriers): one exponentiation alone,
+// full-length exponents, 1024 bits 1.14 -> 0.99 ms, 2048 bits 3.06 -> 2.56, 3072
+// bits 7.82 -> 5.94, 4096 bits 16.9 -> 9.75.  (52-bit digits in tiles through
+// shared memory: 0.87, 3.94, 7.57 and 13.1 ms.)  It does not reach the lane
 // kernels' throughput, so it serves small batches.
 //
-// Supported sizes: n = 32, 64, 96, 128 limbs (1024 .. 4096 bits; (n/4)^2 a
-// multiple of 32 threads); smaller precisions are padded up (any R > N works).
+// Supported sizes: moduli up to 1024, 2048, 3072, 4096 bits in 20, 40, 60, 80
+// digits (any R >= 4 N works).
 #pragma once
 #include "powm_kernel.cuh"
 
 namespace xmpb {
 
-template <int N>
+// LIMBS: the modulus class in limbs (32, 64, 96, 128).
+template <int LIMBS>
 struct CtaShape {
-  static_assert(N % 32 == 0 && N >= 32 && N <= 128, "CTA distribution: 32, 64, 96 or 128 limbs");
-  static constexpr int Q = N / 4;             // tiles per operand
-  static constexpr int THREADS = Q * Q;       // one tile per thread
-  static constexpr int DIAG = 2 * Q - 1;      // anti-diagonals of the tile grid
-  static constexpr int WARPS = THREADS / 32;
+  static_assert(LIMBS % 32 == 0 && LIMBS >= 32 && LIMBS <= 128, "CTA distribution: 32, 64, 96 or 128 limbs");
+  static constexpr int N = LIMBS * 5 / 8;      // digits: 52 N = 32 LIMBS + LIMBS / 2 bits
+  static constexpr int P = LIMBS == 32 ? 4 : 8;  // lanes per column pair
+  static constexpr int K = (N + P - 1) / P;    // products per lane
+  static constexpr int CHUNK = K <= 5 ? K : (K + 1) / 2;  // a warp skips the chunks without terms it needs
+  static constexpr int THREADS = (N * P + 31) / 32 * 32;
+  static constexpr int PAD = 8;  // words around an operand that the lanes beyond it read and do not use
 };
 
-// Column sums of a product, word i = lo[4 + i] + hi[4 + i]: lo takes the low four words of the
-// tiles (anti-diagonal d, word w < 4 -> i = 4 d + w), hi their high four (w >= 4 -> i = 4 d + w);
-// four zero words below word 0 and above word 2n - 1 (never written).
-template <int N>
-struct ColSums {
-  unsigned long long lo[2 * N + 8], hi[2 * N + 8];
-};
-
-// Shared memory of one CTA (the window table follows it, `entries` x N words).
-template <int N>
+// Shared memory of one CTA (the window table follows it, `entries` x N digits).  Operands of role y are stored
+// twice, so that digit (c - i) mod N is at c - i + N.
+template <int LIMBS>
 struct CtaSmem {
-  uint32_t tile[CtaShape<N>::THREADS * 8];  // 8 words per tile
-  ColSums<N> dsum;   // column sums of the current product
-  ColSums<N> dsumT;  // those of T = a b, kept for U = T + m N
-  uint32_t flag[2][32];                     // per warp: carry out with no carry in, all-propagate
-  uint32_t t[2 * N];                        // T = a b
-  uint32_t m[N], u[N];                      // m; the high half of U before its final subtraction
-  uint32_t n[N], np[N];                     // modulus, -N^-1 mod R
-  uint32_t acc[N], x[N], k[N];              // accumulator, operand, a small constant (1 or 2)
-  uint32_t misc[4];
+  static constexpr int N = CtaShape<LIMBS>::N, PAD = CtaShape<LIMBS>::PAD;
+  uint64_t low[2 * N + 2], high[2 * N + 2];  // column sums of the products' low and high halves, from 2 on
+  double pad0[PAD];
+  double n[2 * N + PAD], np[2 * N + PAD];  // modulus, -N^-1 mod R
+  double acc[2 * N + PAD], x[2 * N + PAD];
+  double t[N + PAD], m[N + PAD], one[N + PAD];  // T mod R; m
 };
 
-template <int N>
+template <int LIMBS>
 __host__ __device__ constexpr uint32_t cta_smem_bytes(uint32_t entries) {
-  static_assert(sizeof(CtaSmem<N>) % 16 == 0, "the window table after CtaSmem is read in 16-byte words");
-  return (uint32_t)sizeof(CtaSmem<N>) + entries * N * 4;
+  static_assert(sizeof(CtaSmem<LIMBS>) % 16 == 0, "the window table follows");
+  return (uint32_t)sizeof(CtaSmem<LIMBS>) + (entries * CtaShape<LIMBS>::N + CtaShape<LIMBS>::PAD) * 8;
 }
 
-// v (8 words) = x (4 words) * y (4 words): four row products x y_j (5 words, one carry chain
-// each, independent), added pairwise (rows 0 + 1, rows 2 + 3), then the two halves: a dependent
-// carry path of 4 + 5 + 6 additions instead of one chain through all 16 products.
-__device__ __forceinline__ void cta_row(uint32_t (&r)[5], const uint32_t (&x)[4], uint32_t y) {
-  const uint64_t p0 = mul_wide(x[0], y), p1 = mul_wide(x[1], y), p2 = mul_wide(x[2], y), p3 = mul_wide(x[3], y);
-  r[0] = (uint32_t)p0;
-  r[1] = add_cc((uint32_t)(p0 >> 32), (uint32_t)p1);
-  r[2] = addc_cc((uint32_t)(p1 >> 32), (uint32_t)p2);
-  r[3] = addc_cc((uint32_t)(p2 >> 32), (uint32_t)p3);
-  r[4] = addc((uint32_t)(p3 >> 32), 0u);
-}
-
-// a (6 words) = r (5 words) + q (5 words) * 2^32.
-__device__ __forceinline__ void cta_add_shift(uint32_t (&a)[6], const uint32_t (&r)[5], const uint32_t (&q)[5]) {
-  a[0] = r[0];
-  a[1] = add_cc(r[1], q[0]);
-  a[2] = addc_cc(r[2], q[1]);
-  a[3] = addc_cc(r[3], q[2]);
-  a[4] = addc_cc(r[4], q[3]);
-  a[5] = addc(q[4], 0u);
-}
-
-__device__ __forceinline__ void cta_tile(uint32_t (&v)[8], const uint32_t (&x)[4], const uint32_t (&y)[4]) {
-  uint32_t r0[5], r1[5], r2[5], r3[5], A[6], B[6];
-  cta_row(r0, x, y[0]);
-  cta_row(r1, x, y[1]);
-  cta_row(r2, x, y[2]);
-  cta_row(r3, x, y[3]);
-  cta_add_shift(A, r0, r1);
-  cta_add_shift(B, r2, r3);
-  v[0] = A[0];
-  v[1] = A[1];
-  v[2] = add_cc(A[2], B[0]);
-  v[3] = addc_cc(A[3], B[1]);
-  v[4] = addc_cc(A[4], B[2]);
-  v[5] = addc_cc(A[5], B[3]);
-  v[6] = addc_cc(B[4], 0u);
-  v[7] = addc(B[5], 0u);
-}
-
-// Carry lookahead over W words held one per thread (threads [0, W)): word
-// value z = limb + 2^32 g with g one bit (g = 1 only when limb = 0).  Returns
-// this thread's carry in; *out = the carry out of word W - 1 (every thread).
-// All threads of the CTA call it (one barrier).
-template <int N, int W>
-__device__ __forceinline__ uint32_t cta_carries(CtaSmem<N> &s, uint32_t g, uint32_t p, uint32_t *out) {
-  static_assert(W % 32 == 0 && W <= CtaShape<N>::THREADS, "whole warps of words");
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  constexpr int WW = W / 32;
-  uint32_t G = 0, P = 0;
-  if (warp < WW) {
-    G = __ballot_sync(kFull, g != 0);
-    P = __ballot_sync(kFull, p != 0);
-    if (lane == 0) {
-      s.flag[0][warp] = (uint32_t)((((unsigned long long)P + ((unsigned long long)G << 1)) >> 32) & 1ull);
-      s.flag[1][warp] = P == kFull;
-    }
+// This thread's place: lane p of the group of columns c and N + c; and, as a thread of the first N, digit d.
+template <int LIMBS>
+struct CtaPlace {
+  int c, p, d;
+  int cmin, cmax;   // the columns of this warp
+  __device__ __forceinline__ CtaPlace() {
+    using C = CtaShape<LIMBS>;
+    c = threadIdx.x / C::P;
+    p = threadIdx.x % C::P;
+    d = threadIdx.x;
+    cmin = (threadIdx.x & ~31u) / C::P;
+    cmax = cmin + 32 / C::P - 1;
   }
-  __syncthreads();
-  uint32_t cin = 0, total = 0;
-#pragma unroll
-  for (int k = 0; k < WW; k++) {
-    if (k == warp) cin = total;
-    total = s.flag[0][k] | (s.flag[1][k] & total);
-  }
-  *out = total;
-  const unsigned long long sum = (unsigned long long)P + ((unsigned long long)G << 1) + cin;
-  return (uint32_t)(((sum ^ P) >> lane) & 1ull);
-}
+};
 
-// r = x - y over n words if `take` says so after the fact: with B the borrow
-// out of x - y, r = x - y when force || !B, else r = x.  Returns 1 when it
-// subtracted.  r may alias x.
-template <int N>
-__device__ __forceinline__ uint32_t cta_sub_if(CtaSmem<N> &s, uint32_t *r, const uint32_t *x, const uint32_t *y,
-                                               uint32_t force) {
-  const int i = threadIdx.x;
-  uint32_t xv = 0, d = 0, g = 0, p = 0;
-  if (i < N) {
-    xv = x[i];
-    const uint32_t yv = y[i];
-    d = xv - yv;
-    g = xv < yv;
-    p = xv == yv;
-  }
-  uint32_t borrow;
-  const uint32_t b = cta_carries<N, N>(s, g, p, &borrow);
-  const uint32_t take = force | (borrow ^ 1u);
-  if (i < N) r[i] = take ? d - b : xv;
-  __syncthreads();
-  return take;
-}
+// Sums of this lane's halves: columns c and N + c of a product (and of those added to it).
+struct CtaSums {
+  uint64_t ll, lh, hl, hh;
+};
 
-// ---- the product schedule ---------------------------------------------------------
-// Montgomery's U = T + m N is 0 mod R, so its low half need not be formed: with
-// s_i the column sums of U, the carry out of word i < n - 1 into word i + 1 is
-// exactly hi(s_i) + (lo(s_i) != 0) (the word itself must come out 0), so the
-// carry into word n is c = hi(s_(n-1)) + (lo(s_(n-1)) != 0) and only the words
-// >= n - 1 of U are summed.  T's high half is therefore never resolved either:
-// its raw column sums (dsumT) are added into U's by the same jobs that sum
-// m N's diagonals; only T's low half is resolved (it is m's operand).
-// (Squarings that form only the tiles on and above the tile grid's diagonal,
-// counting the others twice, measured slower with the per-diagonal layout: one
-// 2048-bit exponentiation 4.76 against 4.42 ms -- the tile phase does not get
-// shorter and the diagonal sums pay for the extra predicates.  Sums over a
-// warp-uniform range of tiles instead of all n/4 with predicates, 64-bit
-// uncarried tile columns, and two-word jobs where one-word jobs fit the CTA
-// all measured slower than the form here.)
 enum CtaCols : int { kColsFull = 0, kColsLow = 1, kColsHigh = 2 };
 
-template <int N, int MODE>
-__device__ __forceinline__ void cta_cols(CtaSmem<N> &s, const uint32_t *x, const uint32_t *y,
-                                         ColSums<N> &out) {
-  using C = CtaShape<N>;
-  const int tid = threadIdx.x, ti = tid / C::Q, tj = tid % C::Q;
-  const bool need = MODE == kColsLow ? ti + tj < C::Q : MODE == kColsHigh ? ti + tj >= C::Q - 2 : true;
-  uint32_t v[8];
-  if (need) {
-    const uint4 xa = *reinterpret_cast<const uint4 *>(x + 4 * ti);
-    const uint4 yb = *reinterpret_cast<const uint4 *>(y + 4 * tj);
-    const uint32_t xw[4] = {xa.x, xa.y, xa.z, xa.w}, yw[4] = {yb.x, yb.y, yb.z, yb.w};
-    cta_tile(v, xw, yw);
-    uint4 *tp = reinterpret_cast<uint4 *>(&s.tile[tid * 8]);
-    tp[0] = make_uint4(v[0], v[1], v[2], v[3]);
-    tp[1] = make_uint4(v[4], v[5], v[6], v[7]);
-  }
-  __syncthreads();
-  constexpr int D0 = MODE == kColsHigh ? C::Q - 2 : 0, D1 = MODE == kColsLow ? C::Q : C::DIAG;
-  constexpr bool PAIR = (D1 - D0) * 8 > C::THREADS;  // two words per job when one-word jobs outnumber the threads
-  constexpr int WPJ = PAIR ? 2 : 1, JOBS = (D1 - D0) * 8 / WPJ;
-  for (int j = tid; j < JOBS; j += C::THREADS) {
-    const int d = D0 + j / (8 / WPJ), w = (j % (8 / WPJ)) * WPJ;
-    const int lo = d > C::Q - 1 ? d - (C::Q - 1) : 0, hi = d < C::Q - 1 ? d : C::Q - 1;
-    // all Q loads of the diagonal in flight at once (predicated)
-    unsigned long long a0 = 0, a1 = 0;
-    unsigned long long *o = &(w < 4 ? out.lo : out.hi)[4 + 4 * d + w];
-    const unsigned long long *tt = &(w < 4 ? s.dsumT.lo : s.dsumT.hi)[4 + 4 * d + w];
-    if constexpr (PAIR) {
+// Adds x y's terms x_i y_j, i = p mod P, of columns i + j = c and N + c.  kColsLow: column c only.  kColsHigh:
+// N + c, and c where the warp holds one of the three below N.
+template <int LIMBS, int MODE>
+__device__ __forceinline__ void cta_accumulate(CtaSums &a, const CtaPlace<LIMBS> &me, const double *x,
+                                               const double *y) {
+  using C = CtaShape<LIMBS>;
+  const double *const xp = x + me.p, *const yp = y + C::N + me.c - me.p;
 #pragma unroll
-      for (int t = 0; t < C::Q; t++) {
-        const bool in = t >= lo && t <= hi;
-        const uint2 v = *reinterpret_cast<const uint2 *>(&s.tile[in ? (t * C::Q + (d - t)) * 8 + w : w]);
-        a0 += in ? v.x : 0u;
-        a1 += in ? v.y : 0u;
-      }
-      if constexpr (MODE == kColsHigh) {  // U = T + m N
-        const ulonglong2 t2 = *reinterpret_cast<const ulonglong2 *>(tt);
-        a0 += t2.x;
-        a1 += t2.y;
-      }
-      *reinterpret_cast<ulonglong2 *>(o) = make_ulonglong2(a0, a1);
-    } else {
-      unsigned long long a2 = 0, a3 = 0;  // four accumulators: shorter add chains (4096 bits: 17.9 -> 17.0 ms)
+  for (int k0 = 0; k0 < C::K; k0 += C::CHUNK) {
+    constexpr int L = C::CHUNK;
+    if (C::CHUNK < C::K) {
+      if (MODE == kColsLow && C::P * k0 > me.cmax) break;
+      if (MODE == kColsHigh && C::P * (k0 + L) <= me.cmin + 1 && me.cmax < C::N - 3) continue;
+    }
+    double u[L], v[L], h[L], l[L];
 #pragma unroll
-      for (int t = 0; t < C::Q; t++) {
-        const bool in = t >= lo && t <= hi;
-        const uint32_t v0 = s.tile[in ? (t * C::Q + (d - t)) * 8 + w : w];
-        const uint32_t add = in ? v0 : 0u;
-        if ((t & 3) == 0) a0 += add;
-        else if ((t & 3) == 1) a1 += add;
-        else if ((t & 3) == 2) a2 += add;
-        else a3 += add;
+    for (int k = 0; k < L; k++) {
+      if (k0 + k >= C::K) continue;
+      u[k] = xp[C::P * (k0 + k)];
+      v[k] = yp[-C::P * (k0 + k)];
+    }
+#pragma unroll
+    for (int k = 0; k < L; k++) {
+      if (k0 + k >= C::K) continue;
+      h[k] = __fma_rz(u[k], v[k], kDigHi);
+    }
+#pragma unroll
+    for (int k = 0; k < L; k++) {
+      if (k0 + k >= C::K) continue;
+      l[k] = __fma_rz(u[k], v[k], __dsub_rn(kDigLo, h[k]));
+    }
+#pragma unroll
+    for (int k = 0; k < L; k++) {
+      if (k0 + k >= C::K) continue;
+      const int i = me.p + C::P * (k0 + k);
+      if (i <= me.c) {
+        a.ll += dig_bits(l[k]);
+        a.lh += dig_bits(h[k]);
+      } else if (MODE != kColsLow && (C::N % C::P == 0 || i < C::N)) {
+        a.hl += dig_bits(l[k]);
+        a.hh += dig_bits(h[k]);
       }
-      unsigned long long v = (a0 + a1) + (a2 + a3);
-      if constexpr (MODE == kColsHigh) v += *tt;  // U = T + m N
-      *o = v;
     }
   }
+}
+
+// The groups' sums over their lanes, to s.low and s.high: each step halves the values a lane holds.
+template <int LIMBS, bool BOTH>
+__device__ __forceinline__ void cta_columns(CtaSmem<LIMBS> &s, const CtaPlace<LIMBS> &me, const CtaSums &a) {
+  using C = CtaShape<LIMBS>;
+  const bool odd = me.p & 1;
+  uint64_t v = (odd ? a.lh : a.ll) + __shfl_xor_sync(kFull, odd ? a.ll : a.lh, 1);
+  if (BOTH) {
+    const uint64_t w = (odd ? a.hh : a.hl) + __shfl_xor_sync(kFull, odd ? a.hl : a.hh, 1);
+    const bool up = me.p & 2;
+    v = (up ? w : v) + __shfl_xor_sync(kFull, up ? v : w, 2);
+  } else {
+    v += __shfl_xor_sync(kFull, v, 2);
+  }
+  if (C::P == 8) v += __shfl_xor_sync(kFull, v, 4);
+  if (me.p < (BOTH ? 4 : 2) && me.c < C::N) (odd ? s.high : s.low)[2 + (me.p & 2 ? C::N : 0) + me.c] = v;
   __syncthreads();
 }
 
-// Column sum of product word i (-4 <= i < 2n + 4; 0 outside [0, 2n)).
-template <int N>
-__device__ __forceinline__ unsigned long long cta_ws(const ColSums<N> &c, int i) {
-  return c.lo[4 + i] + c.hi[4 + i];
+// Column j, -1 <= j < 2 N, of one product (of `products`) as a true signed sum.
+template <int LIMBS>
+__device__ __forceinline__ uint64_t cta_column(const CtaSmem<LIMBS> &s, int j, uint32_t products) {
+  constexpr int N = CtaShape<LIMBS>::N;
+  const int pairs = j < N ? j + 1 : 2 * N - 1 - j, below = j < 1 ? 0 : j - 1 < N ? j : 2 * N - j;
+  return s.low[2 + j] + s.high[1 + j] -
+         products * ((uint64_t)pairs * kDigLoBits64 + (uint64_t)below * kDigHiBits64);
 }
 
-// Column sums of words i, i + 1 (i even) with two 16-byte loads.
-template <int N>
-__device__ __forceinline__ void cta_ws2(const ColSums<N> &c, int i, unsigned long long &v0, unsigned long long &v1) {
-  const ulonglong2 a = *reinterpret_cast<const ulonglong2 *>(&c.lo[4 + i]);
-  const ulonglong2 b = *reinterpret_cast<const ulonglong2 *>(&c.hi[4 + i]);
-  v0 = a.x + b.x;
-  v1 = a.y + b.y;
+// The digit of a column: its balanced low 52 bits and the carry of the column below.
+__device__ __forceinline__ double cta_digit(uint64_t v, uint64_t below) {
+  const uint32_t u = (uint32_t)(v >> 32) + 0x80080000u, b = (uint32_t)(below >> 32) + 0x80080000u;  // as dig_settle
+  const double r = __dsub_rn(__hiloint2double((int)((u & 0xfffffu) | 0x43300000u), (int)(uint32_t)v),
+                             0x1p53 + 0x1p51 + 2048.0);
+  return __dadd_rn(r, __hiloint2double(0x43300000, (int)(b >> 20)));
 }
 
-// One warp resolves n words whose column sums sum(j) (j = 0 .. n-1; 0 below)
-// are given, lane l words [lK, lK + K), K = n / 32 (as cta_resolve_warp).
-// SUB: then r = value - N if the value above word n - 1 is set or value >= N.
-template <int N, bool SUB, class Sum, class Sum2>
-__device__ __forceinline__ void cta_resolve_n(CtaSmem<N> &s, Sum sum, Sum2 sum2, uint32_t *out) {
-  constexpr int K = N / 32;
+// Stores digit d of an operand; role y: twice.
+template <int LIMBS>
+__device__ __forceinline__ void cta_put(double *v, int d, double x, bool twice) {
+  v[d] = x;
+  if (twice) v[CtaShape<LIMBS>::N + d] = x;
+}
+
+// out = the low columns of s (+ add at digit 0) mod R.
+template <int LIMBS>
+__device__ __forceinline__ void cta_low_digits(CtaSmem<LIMBS> &s, const CtaPlace<LIMBS> &me, double *out, bool twice,
+                                               uint32_t add = 0) {
+  if (me.d < CtaShape<LIMBS>::N) {
+    const uint64_t v = cta_column(s, me.d, 1), below = cta_column(s, me.d - 1, 1);
+    cta_put<LIMBS>(out, me.d, cta_digit(v + (me.d == 0 ? add : 0u), me.d == 0 ? 0 : below + (me.d == 1 ? add : 0u)),
+                   twice);
+  }
+  __syncthreads();
+}
+
+// out = x y mod R (+ add at digit 0); y of role y.  out may alias x or y.
+template <int LIMBS>
+__device__ __forceinline__ void cta_low_product(CtaSmem<LIMBS> &s, const CtaPlace<LIMBS> &me, double *out, bool twice,
+                                                const double *x, const double *y, uint32_t add = 0) {
+  CtaSums a = {0, 0, 0, 0};
+  cta_accumulate<LIMBS, kColsLow>(a, me, x, y);
+  cta_columns<LIMBS, false>(s, me, a);
+  cta_low_digits(s, me, out, twice, add);
+}
+
+// r = a b R^-1 mod N (|r| <= N); b of role y, r too if `twice`.  r may alias a or b.
+template <int LIMBS>
+__device__ __forceinline__ void mont_cta(CtaSmem<LIMBS> &s, const CtaPlace<LIMBS> &me, double *r, bool twice,
+                                         const double *a, const double *b) {
+  constexpr int N = CtaShape<LIMBS>::N;
+  CtaSums u = {0, 0, 0, 0};
+  cta_accumulate<LIMBS, kColsFull>(u, me, a, b);
+  cta_columns<LIMBS, false>(s, me, u);
+  cta_low_digits(s, me, s.t, false);
+  cta_low_product(s, me, s.m, false, s.t, s.np);
+  cta_accumulate<LIMBS, kColsHigh>(u, me, s.m, s.n);
+  cta_columns<LIMBS, true>(s, me, u);
+  if (me.d < N) {
+    // c = the low half / R: column N - 1 with what column N - 2 carries into it
+    const uint64_t v = cta_column(s, N + me.d, 2), v1 = cta_column(s, N + me.d - 1, 2),
+                   v2 = cta_column(s, N + me.d - 2, 2);
+    cta_put<LIMBS>(r, me.d, cta_digit(v, me.d == 0 ? v1 + (uint64_t)((int64_t)v2 >> 52) : v1), twice);
+  }
+  __syncthreads();
+}
+
+// Digit p of the number with limbs limb(j), balanced (as dig_from_limbs).
+template <class Limb>
+__device__ __forceinline__ double cta_limb_digit(Limb limb, uint32_t p) {
+  const uint32_t o = 52 * p, w = o >> 5, sh = o & 31;
+  uint64_t v = ((uint64_t)limb(w + 1) << 32 | limb(w)) >> sh;
+  if (sh) v |= (uint64_t)limb(w + 2) << (64 - sh);
+  v &= kDigMask;
+  const uint32_t below = o ? (limb((o - 1) >> 5) >> ((o - 1) & 31)) & 1u : 0u;
+  return (double)((int64_t)v - (int64_t)((v >> 51) << 52) + (int64_t)below);
+}
+
+// s.np = -N^-1 mod R by Newton's iteration y <- y (2 + N y), which doubles the correct low digits of y.
+template <int LIMBS>
+__device__ __forceinline__ void cta_neg_inverse(CtaSmem<LIMBS> &s, const CtaPlace<LIMBS> &me, uint64_t inv) {
+  constexpr int N = CtaShape<LIMBS>::N;
+  const auto limb = [&](uint32_t j) { return j == 0 ? (uint32_t)inv : j == 1 ? (uint32_t)(inv >> 32) & 0xfffffu : 0u; };
+  if (threadIdx.x < N) cta_put<LIMBS>(s.np, me.d, me.d ? 0.0 : cta_limb_digit(limb, 0), true);
+  __syncthreads();
+#pragma unroll 1
+  for (int digits = 1; digits < N; digits *= 2) {
+    cta_low_product(s, me, s.m, false, s.n, s.np, 2);
+    cta_low_product(s, me, s.np, true, s.m, s.np);
+  }
+}
+
+// acc = R^2 mod N: warp 0 doubles 2^(bitlen N - 1) exactly on limbs up to 2^(52 N + e), 52 N = e 2^j with e odd
+// (Montgomery form of 2^e), then j Montgomery squarings.  N = 1 gives 0.
+template <int LIMBS>
+__device__ __forceinline__ void cta_r2(CtaSmem<LIMBS> &s, const CtaPlace<LIMBS> &me, const PowmArgs &a, uint32_t em) {
+  constexpr int N = CtaShape<LIMBS>::N, L = LIMBS / 32;
+  constexpr uint32_t bits = 52u * N, j = N == 40 ? 5 : N == 80 ? 6 : 4, e = bits >> j;
+  static_assert(bits == e << j && e % 2 == 1, "52 N = e 2^j");
+  uint32_t *const limbs = reinterpret_cast<uint32_t *>(s.t);
   if (threadIdx.x < 32) {
-    const int l = threadIdx.x, i0 = l * K;
-    unsigned long long sm[K + 2];
-    if constexpr (K % 2 == 0) {
+    Group<32> G;
+    uint32_t n[L], v[L];
+    load_lane_limbs<32, L>(n, a.mod.limbs, a.mod.nlimbs, a.mod.stride, em, G.lane);
+    const uint32_t b = dbitlen<32, L>(G, n);
+    const uint32_t tb = b > 1 ? b - 1 : 0;
 #pragma unroll
-      for (int k = 0; k < K + 2; k += 2) sum2(i0 - 2 + k, sm[k], sm[k + 1]);
-    } else {
+    for (int k = 0; k < L; k++) v[k] = b > 1 && (G.lane * L + k) == (tb >> 5) ? 1u << (tb & 31) : 0u;
+    const uint32_t doublings = b > 1 ? bits + e - tb : 0;
+#pragma unroll 1
+    for (uint32_t d = 0; d < doublings; d++) dmod_double<32, L>(G, v, n, true);
 #pragma unroll
-      for (int k = 0; k < K + 2; k++) sm[k] = sum(i0 - 2 + k);
-    }
-    unsigned long long x[K + 1];
-#pragma unroll
-    for (int k = 0; k <= K; k++) x[k] = (sm[k + 1] & 0xffffffffull) + (sm[k] >> 32);
-    uint32_t limb[K], c = 0, all_ones = 1;
-#pragma unroll
-    for (int k = 0; k < K; k++) {
-      const unsigned long long z = (x[k + 1] & 0xffffffffull) + (x[k] >> 32) + c;
-      limb[k] = (uint32_t)z;
-      c = (uint32_t)(z >> 32);
-      all_ones &= limb[k] == kFull;
-    }
-    const uint32_t G = __ballot_sync(kFull, c != 0), P = __ballot_sync(kFull, all_ones != 0);
-    const unsigned long long cs = (unsigned long long)P + ((unsigned long long)G << 1);
-    uint32_t cin = (uint32_t)(((cs ^ P) >> l) & 1ull);
-#pragma unroll
-    for (int k = 0; k < K; k++) {
-      limb[k] += cin;
-      cin = cin && limb[k] == 0u;
-    }
-    if constexpr (SUB) {
-      const uint32_t top_l = (uint32_t)(sm[K + 1] >> 32) + (uint32_t)(x[K] >> 32);
-      const uint32_t top = __shfl_sync(kFull, top_l, 31) + (uint32_t)((cs >> 32) & 1ull);
-      uint32_t d[K], b = 0, all_zero = 1;
-#pragma unroll
-      for (int k = 0; k < K; k++) {
-        const unsigned long long t = (unsigned long long)limb[k] - s.n[i0 + k] - b;
-        d[k] = (uint32_t)t;
-        b = (uint32_t)(t >> 63);
-        all_zero &= d[k] == 0u;
-      }
-      const uint32_t GB = __ballot_sync(kFull, b != 0), PB = __ballot_sync(kFull, all_zero != 0);
-      const unsigned long long bs = (unsigned long long)PB + ((unsigned long long)GB << 1);
-      uint32_t bin = (uint32_t)(((bs ^ PB) >> l) & 1ull);
-      const bool take = top || !((bs >> 32) & 1ull);
-#pragma unroll
-      for (int k = 0; k < K; k++) {
-        const uint32_t v = d[k] - bin;
-        bin = bin && d[k] == 0u;
-        out[i0 + k] = take ? v : limb[k];
-      }
-    } else {
-#pragma unroll
-      for (int k = 0; k < K; k++) out[i0 + k] = limb[k];
-    }
+    for (int k = 0; k < L; k++) limbs[G.lane * L + k] = v[k];
   }
   __syncthreads();
-}
-
-// r = a b R^-1 mod N (a, b < N; or a, b < R with a b < R N).  r may alias a or b.
-template <int N>
-__device__ __forceinline__ void mont_cta(CtaSmem<N> &s, uint32_t *r, const uint32_t *a, const uint32_t *b) {
-  cta_cols<N, kColsFull>(s, a, b, s.dsumT);
-  cta_resolve_n<N, false>(
-      s, [&](int i) { return cta_ws<N>(s.dsumT, i); },
-      [&](int i, unsigned long long &v0, unsigned long long &v1) { cta_ws2<N>(s.dsumT, i, v0, v1); }, s.t);  // T mod R
-  cta_cols<N, kColsLow>(s, s.t, s.np, s.dsum);
-  cta_resolve_n<N, false>(
-      s, [&](int i) { return cta_ws<N>(s.dsum, i); },
-      [&](int i, unsigned long long &v0, unsigned long long &v1) { cta_ws2<N>(s.dsum, i, v0, v1); }, s.m);  // m
-  cta_cols<N, kColsHigh>(s, s.m, s.n, s.dsum);  // column sums of U from word n - 1 up
-  // Word n - 1 enters as its carry into word n, hi(s) + (lo(s) != 0) (U's low half is 0 mod R),
-  // placed in the high half of a sum whose low half is 0; words below it are 0.
-  const auto low_carry = [](unsigned long long v) {
-    return ((v >> 32) + ((v & 0xffffffffull) != 0ull)) << 32;
-  };
-  cta_resolve_n<N, true>(
-      s,
-      [&](int j) {
-        const unsigned long long v = cta_ws<N>(s.dsum, N + j);
-        return j < -1 ? 0ull : j == -1 ? low_carry(v) : v;
-      },
-      [&](int j, unsigned long long &v0, unsigned long long &v1) {
-        cta_ws2<N>(s.dsum, N + j, v0, v1);
-        if (j < 0) {  // j = -2: words n - 2, n - 1
-          v0 = 0ull;
-          v1 = low_carry(v1);
-        }
-      },
-      r);
-}
-
-// The same as a call: at 4096 bits the constant-schedule kernel's main loop, inlined, overflows
-// the instruction cache (one exponentiation 19.9 ms inlined, 18.5 ms as a call; everywhere else
-// the call measured slower: 2048 bits 3.46 -> 4.00 ms constant-schedule, 3.06 -> 3.95 sliding).
-template <int N>
-__device__ __noinline__ void mont_cta_call(CtaSmem<N> &s, uint32_t *r, const uint32_t *a, const uint32_t *b) {
-  mont_cta<N>(s, r, a, b);
-}
-
-// s.np = -N^-1 mod R by Newton's iteration y <- y (2 + N y), which doubles the
-// correct low words of y = -N^-1 each time (from -N^-1 mod 2^32).
-template <int N>
-__device__ __forceinline__ void cta_neg_inverse(CtaSmem<N> &s) {
-  const int i = threadIdx.x;
-  if (i < N) s.np[i] = i == 0 ? neg_inv32(s.n[0]) : 0u;
+  if (threadIdx.x < N)
+    cta_put<LIMBS>(s.acc, me.d,
+                   cta_limb_digit([&](uint32_t q) { return q < (uint32_t)LIMBS ? limbs[q] : 0u; }, me.d), true);
   __syncthreads();
 #pragma unroll 1
-  for (int words = 1; words < N; words *= 2) {
-    cta_cols<N, kColsLow>(s, s.n, s.np, s.dsum);
-    cta_resolve_n<N, false>(
-        s, [&](int j) { return cta_ws<N>(s.dsum, j) + (j == 0 ? 2ull : 0ull); },
-        [&](int j, unsigned long long &v0, unsigned long long &v1) {
-          cta_ws2<N>(s.dsum, j, v0, v1);
-          v0 += j == 0 ? 2ull : 0ull;
-        },
-        s.m);
-    cta_cols<N, kColsLow>(s, s.np, s.m, s.dsum);
-    cta_resolve_n<N, false>(
-        s, [&](int j) { return cta_ws<N>(s.dsum, j); },
-        [&](int j, unsigned long long &v0, unsigned long long &v1) { cta_ws2<N>(s.dsum, j, v0, v1); }, s.np);
-  }
+  for (uint32_t q = 0; q < j; q++) mont_cta(s, me, s.acc, true, s.acc, s.acc);
 }
 
-// Bit length of s.n (every thread).
-template <int N>
-__device__ __forceinline__ uint32_t cta_bitlen(CtaSmem<N> &s) {
-  const int i = threadIdx.x, lane = i & 31, warp = i >> 5;
-  uint32_t b = 0;
-  if (i < N && s.n[i]) b = (uint32_t)i * 32 + 32 - __clz(s.n[i]);
-  if (warp < N / 32) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) b = max(b, __shfl_xor_sync(kFull, b, o));
-    if (lane == 0) s.flag[0][warp] = b;
-  }
-  __syncthreads();
-  uint32_t m = 0;
-  for (int k = 0; k < N / 32; k++) m = max(m, s.flag[0][k]);
-  __syncthreads();
-  return m;
-}
-
-// v <- 2 v mod N for v < N.
-template <int N>
-__device__ __forceinline__ void cta_double(CtaSmem<N> &s, uint32_t *v) {
-  const int i = threadIdx.x;
-  uint32_t w = 0, top = 0;
-  if (i < N) {
-    w = (v[i] << 1) | (i ? v[i - 1] >> 31 : 0u);
-    top = v[N - 1] >> 31;
-  }
-  __syncthreads();
-  if (i < N) v[i] = w;
-  __syncthreads();
-  cta_sub_if<N>(s, v, v, s.n, top);
-}
-
-// acc = R^2 mod N (R = 2^(32 n)): 2^(bitlen N - 1) doubled up to 2^(32n + e)
-// with 32n = e 2^j (e odd), then j Montgomery squarings, each doubling the
-// exponent above R.  N = 1 gives 0.
-template <int N>
-__device__ __forceinline__ void cta_r2(CtaSmem<N> &s, uint32_t *acc) {
-  constexpr uint32_t bits = 32u * N;
-  constexpr uint32_t j = bits == 1024 ? 10 : bits == 2048 ? 11 : bits == 3072 ? 10 : 12;
-  constexpr uint32_t e = bits >> j;
-  const uint32_t b = cta_bitlen<N>(s);
-  const int i = threadIdx.x;
-  const uint32_t tb = b > 1 ? b - 1 : 0;
-  if (i < N) acc[i] = (b > 1 && (uint32_t)i == (tb >> 5)) ? (1u << (tb & 31)) : 0u;
-  __syncthreads();
-  if (b <= 1) return;
-#pragma unroll 1
-  for (uint32_t d = 0; d < bits + e - tb; d++) cta_double<N>(s, acc);
-#pragma unroll 1
-  for (uint32_t q = 0; q < j; q++) mont_cta<N>(s, acc, acc, acc);
-}
-
-// Copies n words within shared memory (every thread calls it).
-template <int N>
-__device__ __forceinline__ void cta_copy(uint32_t *dst, const uint32_t *src) {
-  if (threadIdx.x < N) dst[threadIdx.x] = src[threadIdx.x];
+// Copies N digits within shared memory, to an operand of role y (every thread calls it).
+template <int LIMBS>
+__device__ __forceinline__ void cta_copy(double *dst, const double *src) {
+  if (threadIdx.x < CtaShape<LIMBS>::N) cta_put<LIMBS>(dst, threadIdx.x, src[threadIdx.x], true);
   __syncthreads();
 }
 
@@ -447,41 +290,46 @@ __device__ __forceinline__ void cta_copy(uint32_t *dst, const uint32_t *src) {
 // precision (the same schedule for every exponent).  The window table
 // (sliding: slot 0 = Mont(1), slot j = Mont(x^(2j - 1)); fixed: slot e =
 // Mont(x^e)) is in shared memory after the CtaSmem block.
-template <int N, bool CT>
-__global__ void __launch_bounds__(CtaShape<N>::THREADS) powm_cta_kernel(PowmArgs a) {
+template <int LIMBS, bool CT>
+__global__ void __launch_bounds__(CtaShape<LIMBS>::THREADS, 1) powm_cta_kernel(PowmArgs a) {
+  using C = CtaShape<LIMBS>;
+  constexpr int N = C::N;
   extern __shared__ uint4 cta_dyn_smem[];
-  CtaSmem<N> &s = *reinterpret_cast<CtaSmem<N> *>(cta_dyn_smem);
-  uint32_t *table = reinterpret_cast<uint32_t *>(cta_dyn_smem) + sizeof(CtaSmem<N>) / 4;
+  CtaSmem<LIMBS> &s = *reinterpret_cast<CtaSmem<LIMBS> *>(cta_dyn_smem);
+  double *table = reinterpret_cast<double *>(reinterpret_cast<char *>(cta_dyn_smem) + sizeof(CtaSmem<LIMBS>));
+  const CtaPlace<LIMBS> me;
   const uint32_t inst = a.start + blockIdx.x;
-  const int i = threadIdx.x;
+  const uint32_t i = threadIdx.x;
   const uint32_t eb = in_element(a.base, inst), ee = in_element(a.exp, inst), em = in_element(a.mod, inst);
+  const auto mod_limb = [&](uint32_t j) { return load_limb(a.mod.limbs, a.mod.nlimbs, a.mod.stride, em, j); };
+  for (uint32_t w = i; w < sizeof(CtaSmem<LIMBS>) / 8; w += C::THREADS) reinterpret_cast<uint64_t *>(&s)[w] = 0;
+  __syncthreads();
   if (i < N) {
-    s.n[i] = load_limb(a.mod.limbs, a.mod.nlimbs, a.mod.stride, em, (uint32_t)i);
-    s.x[i] = load_limb(a.base.limbs, a.base.nlimbs, a.base.stride, eb, (uint32_t)i);
-    s.k[i] = i == 0 ? 1u : 0u;
-  }
-  {
-    unsigned long long *z = &s.dsum.lo[0];  // dsum and dsumT: 4 arrays of 2n + 8 words, contiguous
-    for (int w = i; w < 4 * (2 * N + 8); w += CtaShape<N>::THREADS) z[w] = 0ull;
+    cta_put<LIMBS>(s.n, i, cta_limb_digit(mod_limb, i), true);
+    cta_put<LIMBS>(
+        s.x, i,
+        cta_limb_digit([&](uint32_t j) { return load_limb(a.base.limbs, a.base.nlimbs, a.base.stride, eb, j); }, i),
+        true);
+    s.one[i] = i == 0 ? 1.0 : 0.0;
   }
   __syncthreads();
-  // x may be >= N (any base below R): x mod N comes out of Mont(x, R^2) = x R mod N
-  cta_neg_inverse<N>(s);
-  cta_r2<N>(s, s.acc);
-  uint32_t *const one = s.k;  // cta_neg_inverse left 2 in word 0: reset below
-  if (i < N) one[i] = i == 0 ? 1u : 0u;
-  __syncthreads();
+  // x may be >= N (any base below R / 4): x mod N comes out of Mont(x, R^2) = x R mod N
+  cta_neg_inverse(s, me, dig_neg_inv(mod_limb(0), mod_limb(1)));
+  cta_r2(s, me, a, em);
   const uint32_t W = a.window;
   const bool sliding = !CT;
   // table
-  uint32_t *t1 = table + N;
-  mont_cta<N>(s, t1, s.x, s.acc);  // Mont(x)
-  mont_cta<N>(s, table, s.acc, one);  // Mont(1) = R mod N
+  double *t1 = table + N;
+  mont_cta(s, me, t1, false, s.x, s.acc);       // Mont(x)
+  mont_cta(s, me, table, false, s.one, s.acc);  // Mont(1) = R mod N
+  cta_copy<LIMBS>(s.x, t1);
   if (sliding) {
-    mont_cta<N>(s, s.x, t1, t1);  // Mont(x^2)
-    for (uint32_t j = 2; j <= (1u << (W - 1)); j++) mont_cta<N>(s, table + j * N, table + (j - 1) * N, s.x);
+    mont_cta(s, me, s.x, true, t1, s.x);  // Mont(x^2)
+#pragma unroll 1
+    for (uint32_t j = 2; j <= (1u << (W - 1)); j++) mont_cta(s, me, table + j * N, false, table + (j - 1) * N, s.x);
   } else {
-    for (uint32_t j = 2; j < (1u << W); j++) mont_cta<N>(s, table + j * N, table + (j - 1) * N, t1);
+#pragma unroll 1
+    for (uint32_t j = 2; j < (1u << W); j++) mont_cta(s, me, table + j * N, false, table + (j - 1) * N, s.x);
   }
   if (sliding) {
     // scan from the exponent's top bit
@@ -493,7 +341,7 @@ __global__ void __launch_bounds__(CtaShape<N>::THREADS) powm_cta_kernel(PowmArgs
         break;
       }
     }
-    cta_copy<N>(s.acc, table);  // Mont(1)
+    cta_copy<LIMBS>(s.acc, table);  // Mont(1)
     ExpCursor cur;
     cursor_init(cur, a.exp, ee, top);
     uint32_t sq, idx;
@@ -502,35 +350,50 @@ __global__ void __launch_bounds__(CtaShape<N>::THREADS) powm_cta_kernel(PowmArgs
       const bool more = next_window(a.exp, ee, cur, W, &sq, &idx);
       if (first && more) {
         // the accumulator is Mont(1): skip the squarings and take the first window's entry
-        cta_copy<N>(s.acc, table + idx * N);
+        cta_copy<LIMBS>(s.acc, table + idx * N);
         first = false;
         continue;
       }
-      for (uint32_t q = 0; q < sq; q++) mont_cta<N>(s, s.acc, s.acc, s.acc);
+      // sq squarings and, unless the exponent ends, the window's entry: one product in the code
+#pragma unroll 1
+      for (uint32_t q = 0; q < sq + (more ? 1u : 0u); q++)
+        mont_cta(s, me, s.acc, true, q < sq ? s.acc : table + idx * N, s.acc);
       if (!more) break;
-      mont_cta<N>(s, s.acc, s.acc, table + idx * N);
     }
   } else {
     const uint32_t nwin = (a.exp.nlimbs * 32 + W - 1) / W;
-    cta_copy<N>(s.acc, table + exp_window(a.exp, ee, (nwin - 1) * W, W) * N);
+    cta_copy<LIMBS>(s.acc, table + exp_window(a.exp, ee, (nwin - 1) * W, W) * N);
 #pragma unroll 1
     for (int32_t wi = (int32_t)nwin - 2; wi >= 0; wi--) {
       const uint32_t win = exp_window(a.exp, ee, (uint32_t)wi * W, W);
 #pragma unroll 1
-      for (uint32_t q = 0; q < W; q++) {
-        if constexpr (N == 128) mont_cta_call<N>(s, s.acc, s.acc, s.acc);
-        else mont_cta<N>(s, s.acc, s.acc, s.acc);
-      }
-      if constexpr (N == 128) mont_cta_call<N>(s, s.acc, s.acc, table + win * N);
-      else mont_cta<N>(s, s.acc, s.acc, table + win * N);
+      for (uint32_t q = 0; q <= W; q++) mont_cta(s, me, s.acc, true, q < W ? s.acc : table + win * N, s.acc);
     }
   }
-  mont_cta<N>(s, s.acc, s.acc, one);
+  mont_cta(s, me, s.acc, false, s.one, s.acc);
+  // into [0, N) on warp 0, then to limbs
+  constexpr int D = (N + 31) / 32;
+  uint64_t *const st = reinterpret_cast<uint64_t *>(s.t);
+  if (i < 32) {
+    Group<32> G;
+    double v[D], n[D];
+#pragma unroll
+    for (int k = 0; k < D; k++) {
+      const uint32_t p = G.lane * D + k;
+      v[k] = p < N ? s.acc[p] : 0.0;
+      n[k] = p < N ? s.n[p] : 0.0;
+    }
+    int64_t c[D];
+    dig_canon<32, D>(G, c, v, n);
+#pragma unroll
+    for (int k = 0; k < D; k++)
+      if (G.lane * D + k < N) st[G.lane * D + k] = (uint64_t)c[k];
+  }
+  __syncthreads();
   const uint32_t o = out_element(a.out, inst);
-  if (o < a.out.count && i < N && (uint32_t)i < a.out.nlimbs) limb_ref(a.out.limbs, a.out.stride, o, (uint32_t)i) = s.acc[i];
-  // output words above n (a wider output array) are zero
-  for (uint32_t w = N + i; w < a.out.nlimbs && o < a.out.count; w += CtaShape<N>::THREADS)
-    limb_ref(a.out.limbs, a.out.stride, o, w) = 0u;
+  if (o < a.out.count)
+    for (uint32_t g = i; g < div_up(a.out.nlimbs, 4); g += C::THREADS)
+      store_group(a.out.limbs, a.out.nlimbs, a.out.stride, o, g, dig_group(st, N, g));
 }
 
 }  // namespace xmpb

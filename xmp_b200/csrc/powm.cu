@@ -45,18 +45,18 @@ int window_for_bits(uint32_t exp_bits, bool sliding) {
 
 bool powm_cta_preferred(uint32_t nlimbs, uint32_t count, uint32_t sm_count) {
   const uint32_t limbs = powm_cta_limbs(nlimbs);
-  // Up to 512 bits the smallest CTA (1024-bit operands) pads too much: one instance measured 0.27 /
-  // 0.46 / 0.69 ms at 64 / 256 / 512 bits against 0.017 / 0.18 / 0.61 ms on the lane kernels; from
-  // 544 bits on it is faster at every measured size (544: 0.72 vs 1.20 ms, 1056: 1.82 vs 2.97,
-  // 1536: 2.42 vs 4.20, 2080: 5.54 vs 11.0, 3104: 13.9 vs 23.4, 4096: 17.7 vs 30.5 ms).
+  // Up to 512 bits the smallest CTA (1024-bit operands) pads too much: it ties with the lane kernels at 512
+  // bits (0.55 ms for 148 instances, 0.59 ms for 296, vs 0.59 ms) and loses below (384 bits 0.44 ms vs 0.48 on 8
+  // lanes, less on fewer).  From 544 bits on it is faster alone at every measured size (544: 0.57 vs 1.11 ms on 8 x 4,
+  // 1056: 1.40 vs 2.86, 1536: 1.97 vs 4.04, 2048: 2.56 vs 7.6, 3072: 5.94 vs 15.6, 4096: 9.7 vs 29.3 ms).
   if (!limbs || nlimbs <= 16) return false;
   // A CTA per instance runs it near its lone latency while the SMs hold the batch; the lane kernels
-  // need thousands of instances before their throughput beats that.  Measured on B200 through
-  // xmpIntegersPowm (full-length exponents), CTA vs the lane kernel at 148 / 296 / 444 / 592 / 888 /
-  // 1184 instances: 768 bits -/-/-/1.12/1.36 vs 1.64/1.16 ms; 1024 bits 1.15/1.17/1.36/1.39/1.71/2.10
-  // vs 2.13 ms; 1280 bits 2.90 (296), 4.81 (370) vs 3.57 ms; 1536 bits 2.43/3.37/5.60 vs 4.21 ms;
-  // 1792 bits 3.84/6.37 (444) vs 7.15 ms; 2048 bits 3.08/4.30/7.15/8.57 vs 8.12 ms; 3072 bits
-  // 7.84/15.7 vs 16.0 ms; 4096 bits 17.8/35.6 vs 30.6 ms.
+  // need thousands of instances before their throughput beats that.  Measured on B200 (full-length
+  // exponents), CTA at 148 / 296 / 444 / 592 / 888 instances vs the best lane kernel: 768 bits
+  // 0.78/0.84/0.91/0.97/1.20 vs 1.11 ms; 1024 bits 0.99/1.07/1.17/1.25/1.54 vs 2.03 ms; 1536 bits
+  // 1.98/2.51/4.35 vs 4.03 ms; 2048 bits 2.58/3.27/5.68/6.52 vs 7.7 ms; 3072 bits 5.98/11.9 vs 15.6 ms;
+  // 4096 bits 9.8/19.5 vs 29.5 ms.  The limits are the ones that callers of the default have had: above
+  // 1024 bits a second or fourth CTA per SM would gain as well.
   uint32_t per_sm = 1;
   if (limbs == 32) per_sm = nlimbs > 24 ? 6 : 4;
   else if (limbs == 64) per_sm = nlimbs > 48 ? 3 : 2;
