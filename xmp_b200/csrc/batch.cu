@@ -217,37 +217,40 @@ xmpError_t XMPAPI xmpPowmBatchPlanCreate(xmpHandle_t h, const xmpPowmBatchItem_t
     }
   }
   // ---- configurations and grids ----
-  // Every bin gets a full persistent grid (SMs x resident CTAs) and all bins
-  // are launched at once, longest instances first: the block scheduler runs
-  // them back to back at full width and fills each bin's tail with the next
-  // bin's CTAs, with no work estimate to get wrong.  Lanes and limbs are the
-  // tuner's choice at a saturating batch (an exact tuned entry for the bin's
-  // own shape wins); the window follows the exponent length.
-  const uint32_t kSaturated = 1u << 16;
+  // Every bin gets a full persistent grid (SMs x resident CTAs) and all bins are launched at once, longest
+  // instances first: the block scheduler runs them back to back at full width and fills each bin's tail with
+  // the next bin's CTAs.  A bin's kernel (an exact tuned entry for its own shape wins) is the one that would
+  // take its instances through soonest alone: the most efficient kernel of a full GPU leaves a bin of few long
+  // instances running when everything else is done (8,192 instances of 1024 to 4096 bits: 65 ms with
+  // every bin's kernel chosen for 65,536 instances, 55 with this rule, 53.8 with the best of 200 assignments).
   for (auto &b : p->bins) {
     PowmConfig c;
     int src = 0;
-    bool exact = tuner_lookup(h, xmpTunePowm, b.nlimbs * 32, b.exp_bits, b.count, &src) >= 0 && src == 1 &&
-                 tuner_lookup_powm(h, b.nlimbs, b.exp_bits, b.count, &c) && c.dist == kDistLanes;
-    if (!exact) {
-      bool tuned = tuner_lookup_powm(h, b.nlimbs, b.exp_bits, std::max(b.count, kSaturated), &c) &&
-                   c.dist == kDistLanes;
-      if (!tuned)
-        c = powm_default_config(b.nlimbs, b.exp_bits, std::max(b.count, kSaturated), xmpAlgorithmDefault,
-                                h->sm_count);
-      c.window = window_for_bits(b.exp_bits, c.dist != kDistDigit && powm_sliding(c.tpi, c.limbs));
+    if (tuner_lookup(h, xmpTunePowm, b.nlimbs * 32, b.exp_bits, b.count, &src) >= 0 && src == 1 &&
+        tuner_lookup_powm(h, b.nlimbs, b.exp_bits, b.count, &c) && c.dist == kDistLanes) {
+      b.cfg = c;
+      continue;
     }
-    if (c.dist == kDistDigit) {
-      // prefer any register kernel that holds the precision; else digit-serial after the join
-      PowmConfig r = powm_default_config(b.nlimbs, b.exp_bits, b.count, xmpAlgorithmDistributedMP, h->sm_count);
-      if (r.tpi) c = r;
-      else b.serial = true;
+    double best = 1e300;
+    for (const auto &e : powm_registry()) {
+      if ((uint32_t)e.tpi * e.limbs < b.nlimbs) continue;
+      const double t = powm_shape_cycles(e.tpi, e.limbs, b.count, h->sm_count);
+      if (t >= best) continue;
+      best = t;
+      b.cfg = PowmConfig();
+      b.cfg.tpi = e.tpi;
+      b.cfg.limbs = e.limbs;
+      b.cfg.window = window_for_bits(b.exp_bits, powm_sliding(e.tpi, e.limbs));
     }
-    b.cfg = c;
-    if (!b.serial) {
-      b.k = powm_find(c.tpi, c.limbs);
-      if (!b.k) return fail(xmpErrorUnsupported);
+  }
+  for (auto &b : p->bins) {
+    if (!b.cfg.tpi) {  // above every register kernel: digit-serial after the join
+      b.cfg = powm_default_config(b.nlimbs, b.exp_bits, b.count, xmpAlgorithmDefault, h->sm_count);
+      b.serial = true;
+      continue;
     }
+    b.k = powm_find(b.cfg.tpi, b.cfg.limbs);
+    if (!b.k) return fail(xmpErrorUnsupported);
   }
   // launch order: longest instances (work per instance) first
   std::stable_sort(p->bins.begin(), p->bins.end(), [](const BatchBin &x, const BatchBin &y) {
@@ -257,8 +260,6 @@ xmpError_t XMPAPI xmpPowmBatchPlanCreate(xmpHandle_t h, const xmpPowmBatchItem_t
   for (auto &b : p->bins) {
     if (b.serial) continue;
     int occ = 0;
-    if (b.k->smem > 48 * 1024)
-      cudaFuncSetAttribute(b.k->batch_fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)b.k->smem);
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, b.k->batch_fn, 128, b.k->smem);
     occ = std::max(occ, 1);
     const uint32_t per_item = 32 / b.cfg.tpi;
