@@ -120,6 +120,7 @@ struct _xmpHandle_t {
   xmpExecutionPolicy_t policy;
   _xmpExecutionPolicy_t default_policy;
   void *tuner;  // xmpb::TunerState*, created lazily
+  void *mailbox;  // xmpb::kMailboxBytes of mapped host memory, small exports land there (null: not to be had)
 };
 
 // Integer array: only the interleaved layout is kept on the device.
@@ -161,7 +162,11 @@ xmpError_t ensure_tmp_out(xmpHandle_t h, size_t bytes);
 size_t scratch_limit(xmpHandle_t h);
 
 // True when `p` is host memory the device cannot address directly (pageable or unknown).
-bool is_host_pointer(const void *p);
+// *pageable (optional): memory that no stream operation writes behind the host's back.
+bool is_host_pointer(const void *p, bool *pageable = nullptr);
+
+// Rows that a synchronous import passes as kernel arguments, and an export takes through the mailbox.
+constexpr size_t kSmallImportBytes = 3584, kMailboxBytes = 64 << 10;
 
 inline ArrayView view_in(xmpIntegers_t x, const uint32_t *index = nullptr, uint32_t index_count = 0) {
   ArrayView v;

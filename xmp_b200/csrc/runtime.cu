@@ -58,13 +58,15 @@ xmpError_t ensure_tmp_out(xmpHandle_t h, size_t bytes) {
   return check_cuda();
 }
 
-bool is_host_pointer(const void *p) {
+bool is_host_pointer(const void *p, bool *pageable) {
   cudaPointerAttributes attr;
   cudaError_t e = cudaPointerGetAttributes(&attr, p);
   if (e != cudaSuccess) {
     cudaGetLastError();
+    if (pageable) *pageable = false;
     return true;
   }
+  if (pageable) *pageable = attr.type == cudaMemoryTypeUnregistered;
   return !(attr.type == cudaMemoryTypeDevice || attr.type == cudaMemoryTypeManaged);
 }
 
@@ -346,6 +348,25 @@ __global__ void interleaved_to_compact(const uint32_t *__restrict__ limbs, uint3
   }
 }
 
+// A few native rows passed by value: a synchronous import of pageable rows up to kSmallImportBytes needs no
+// copy in front of its kernel (256-bit rows x 100, two imports, an add and an export: 59 -> 52 us together
+// with the export's mailbox).  The kernel's parameters are 4 KB; larger rows gain nothing from it.
+struct SmallRows {
+  uint32_t w[kSmallImportBytes / 4];
+};
+__global__ void small_rows_to_interleaved(const __grid_constant__ SmallRows rows, uint32_t *__restrict__ limbs,
+                                          uint32_t nlimbs, uint32_t stride, uint32_t count) {
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x, g = blockIdx.y;
+  if (i >= count) return;
+  const uint32_t at = i * nlimbs + 4 * g, left = nlimbs - 4 * g;
+  uint4 v;
+  v.x = rows.w[at];
+  v.y = left > 1 ? rows.w[at + 1] : 0;
+  v.z = left > 2 ? rows.w[at + 2] : 0;
+  v.w = left > 3 ? rows.w[at + 3] : 0;
+  reinterpret_cast<uint4 *>(limbs)[(size_t)g * stride + i] = v;
+}
+
 // Indexed copy between arrays of equal precision (xmpReorder_compact_kernel, src/xmp.cu:693-716).
 __global__ void reorder_kernel(const uint32_t *__restrict__ in, uint32_t in_stride, uint32_t in_count,
                                const uint32_t *in_index, uint32_t in_index_count, uint32_t *__restrict__ out,
@@ -395,6 +416,11 @@ xmpError_t XMPAPI xmpHandleCreateWithMemoryFunctions(xmpHandle_t *handle, xmpAll
   h->memory_size = prop.totalGlobalMem;
   h->arch = prop.major * 10 + prop.minor;
   h->sm_count = prop.multiProcessorCount;
+  // Mapped under unified addressing: kernels use the host pointer.  Without it exports take a device copy.
+  if (cudaHostAlloc(&h->mailbox, kMailboxBytes, cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess) {
+    h->mailbox = nullptr;
+    cudaGetLastError();
+  }
   // Configuration choices start from the compiled-in learned selector; if it cannot be
   // loaded (e.g. the caller's allocator refuses), the built-in heuristic stays in charge.
   int members = 0;
@@ -413,6 +439,7 @@ xmpError_t XMPAPI xmpHandleDestroy(xmpHandle_t handle) {
   cudaStreamSynchronize(handle->stream);
   if (handle->scratch) handle->df(handle->scratch);
   if (handle->tmp_out) handle->df(handle->tmp_out);
+  if (handle->mailbox) cudaFreeHost(handle->mailbox);
   tuner_destroy(handle);
   xmpFreeFunc hf = handle->hf;
   hf(handle);
@@ -637,7 +664,25 @@ static xmpError_t import_internal(xmpHandle_t handle, xmpIntegers_t out, uint32_
   const uint32_t *gather = policy->indices[0];
   uint32_t rows = 0xffffffffu;
   const void *src = in;
-  if (is_host_pointer(in)) {
+  bool pageable = false;
+  if (is_host_pointer(in, &pageable)) {
+    // Only where the host may read the rows now: the asynchronous form may be captured and replayed, pinned
+    // rows may be the target of a copy of any stream, and work on this one may yet write pageable rows.
+    bool now = !async && pageable && bytes <= kSmallImportBytes && size == 4 && order == -1 &&
+               endian == native_endian() && nails == 0 && gather == nullptr;
+    if (now && cudaStreamQuery(handle->stream) != cudaSuccess) {
+      cudaGetLastError();
+      now = false;
+    }
+    if (now) {
+      if (bytes > scratch_limit(handle)) return xmpErrorIncreaseScratchLimit;  // as the staged copy below
+      SmallRows r;
+      memcpy(r.w, in, bytes);
+      small_rows_to_interleaved<<<dim3(grid_for(count, 128), out->ngroups), 128, 0, handle->stream>>>(
+          r, out->limbs, out->nlimbs, out->stride, count);
+      cudaStreamSynchronize(handle->stream);
+      return check_cuda();
+    }
     rows = count;
     xmpError_t e = ensure_scratch(handle, bytes);
     if (e != xmpErrorSuccess) return e;
@@ -697,10 +742,17 @@ static xmpError_t export_internal(xmpHandle_t handle, void *out, uint32_t *words
   uint32_t w = (uint32_t)(in->nlimbs * 4 / size);
   const uint32_t *scatter = policy->indices[0];
   size_t bytes = (size_t)count * w * size;
-  bool host = is_host_pointer(out);
+  bool pageable = false;
+  bool host = is_host_pointer(out, &pageable);
   void *dst = out;
   uint32_t rows = 0xffffffffu;
-  if (host) {
+  // A small synchronous export is written straight to mapped host memory and copied out after the wait.
+  const bool mail = host && !async && pageable && handle->mailbox && bytes <= kMailboxBytes && scatter == nullptr;
+  if (mail) {
+    if (bytes > scratch_limit(handle)) return xmpErrorIncreaseScratchLimit;  // as the staged copy
+    rows = count;
+    dst = handle->mailbox;
+  } else if (host) {
     rows = count;
     xmpError_t e = ensure_scratch(handle, bytes);
     if (e != xmpErrorSuccess) return e;
@@ -734,6 +786,12 @@ static xmpError_t export_internal(xmpHandle_t handle, void *out, uint32_t *words
         default: export_kernel<uint64_t><<<grid, block, 0, handle->stream>>>(in->limbs, in->nlimbs, in->stride, (uint64_t *)dst, a); break;
       }
     }
+  }
+  if (mail) {
+    if (cudaStreamSynchronize(handle->stream) != cudaSuccess) return xmpErrorCuda;
+    memcpy(out, dst, bytes);
+    if (words_out) *words_out = w;
+    return check_cuda();
   }
   if (host) {
     if (cudaMemcpyAsync(out, dst, bytes, cudaMemcpyDeviceToHost, handle->stream) != cudaSuccess) return xmpErrorCuda;
