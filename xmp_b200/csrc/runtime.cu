@@ -259,7 +259,7 @@ __global__ void __launch_bounds__(256) wire_tile_kernel(U *__restrict__ wire, ui
   }
 }
 
-constexpr uint64_t kDirectBytes = 8u << 20;
+constexpr uint64_t kDirectBytes = 16u << 20;
 static bool wire_native(const WireArgs &a, size_t size) {
   return size == 4 && a.order == -1 && !a.swap && a.nails == 0 && a.index == nullptr;
 }
@@ -270,6 +270,10 @@ template <bool IMPORT>
 static bool wire_tiles(void *wire, xmpIntegers_t x, size_t size, const WireArgs &a, cudaStream_t stream) {
   const uint64_t bytes = (uint64_t)a.words * size;
   if (bytes != (uint64_t)x->nlimbs * 4) return false;
+  // Few words: a tile's two steps in few CTAs take longer than a thread per word (imports and exports of 2080
+  // bits x 164 in bytes 28 us on words, 37 on tiles; 4096 x 868 in 16-bit words 49 / 56, 768 x 10,198 in 64-bit
+  // words 63 / 70; above, 4096 x 1,487 in bytes 68 / 57, 2048 x 4,737 in 16-bit words 85 / 81).
+  if (!wire_native(a, size) && (uint64_t)a.words * a.count <= 1u << 19 && bytes * a.count <= 1u << 20) return false;
   WirePerm w;
   const bool rev = a.order == 1, swap = a.swap && size > 1;
   w.reverse = rev;
@@ -290,6 +294,8 @@ static bool wire_tiles(void *wire, xmpIntegers_t x, size_t size, const WireArgs 
   w.mask[1] = (uint32_t)(mm >> 32);
   const bool vec = x->nlimbs % 4 == 0 && (uintptr_t)wire % 16 == 0;
   if (!vec && (size == 8 || (uintptr_t)wire % 4 != 0)) return false;
+  // Single limbs come in faster a thread per word up to 4 MB (320 bits in 16-bit words, 1.5 MB: 5.3 / 6.9 us).
+  if (IMPORT && !vec && bytes * a.count <= 4u << 20) return false;
   const uint32_t ng = x->ngroups < kTileGroups ? x->ngroups : kTileGroups;
   uint32_t lg = 5;
   while ((ng << (lg + 1)) <= kTileUnits) lg++;
@@ -306,10 +312,11 @@ static bool wire_tiles(void *wire, xmpIntegers_t x, size_t size, const WireArgs 
 }
 
 // Native rows (compact uint32, no index) <-> interleaved groups directly, one uint4 per thread, for small
-// arrays: up to 8 MB the L2 joins the pieces of a row's sectors and a launch costs less than the tile's two
+// arrays: up to 16 MB the L2 joins the pieces of a row's sectors and a launch costs less than the tile's two
 // steps (256-bit rows x 100, three of these and an add with their copies: 59.1 us against 61.6 with tiles;
-// 2048 bits x 16,384: 7 us both ways).  Rows of a partial group come in this way at every size (1056 bits x
-// 65,536: 8.4 against 10.9 us).
+// 384 bits, 16 MB: import 14.7 / 15.5 us, export 14.6 / 15.4; beyond, 2048 bits, 32 MB: 21.5 / 19.8 and 23.0 /
+// 17.2 us, 128 MB: 86 / 56 and 164 / 51 us).  Rows of one group, and rows of a partial group on their way in, take
+// this way at every size (128 bits, 128 MB: 49 / 56 and 49 / 51 us; 1056 bits x 65,536 in: 8.4 against 10.9 us).
 // `vec` (128-bit row access) requires nlimbs % 4 == 0 and a 16-byte aligned buffer.
 __global__ void compact_to_interleaved(const uint32_t *__restrict__ in, uint32_t *__restrict__ limbs,
                                        uint32_t nlimbs, uint32_t stride, uint32_t count, bool vec) {
@@ -699,7 +706,7 @@ static xmpError_t import_internal(xmpHandle_t handle, xmpIntegers_t out, uint32_
   a.index = gather;
   a.index_count = policy->indices_count[0];
   a.rows = rows;
-  if (wire_native(a, size) && (bytes <= kDirectBytes || out->nlimbs % 4 != 0)) {
+  if (wire_native(a, size) && (bytes <= kDirectBytes || out->ngroups == 1 || out->nlimbs % 4 != 0)) {
     dim3 block(128), grid(grid_for(count, 128), out->ngroups);
     bool vec = (out->nlimbs % 4 == 0) && ((uintptr_t)src % 16 == 0);
     compact_to_interleaved<<<grid, block, 0, handle->stream>>>((const uint32_t *)src, out->limbs, out->nlimbs,
@@ -746,8 +753,10 @@ static xmpError_t export_internal(xmpHandle_t handle, void *out, uint32_t *words
   bool host = is_host_pointer(out, &pageable);
   void *dst = out;
   uint32_t rows = 0xffffffffu;
-  // A small synchronous export is written straight to mapped host memory and copied out after the wait.
-  const bool mail = host && !async && pageable && handle->mailbox && bytes <= kMailboxBytes && scatter == nullptr;
+  // A small synchronous export of native rows is written straight to mapped host memory and copied out after
+  // the wait (other formats leave in pieces too small for the bus).
+  const bool mail = host && !async && pageable && handle->mailbox && bytes <= kMailboxBytes && scatter == nullptr &&
+                    size == 4 && order == -1 && endian == native_endian() && nails == 0;
   if (mail) {
     if (bytes > scratch_limit(handle)) return xmpErrorIncreaseScratchLimit;  // as the staged copy
     rows = count;
@@ -772,7 +781,7 @@ static xmpError_t export_internal(xmpHandle_t handle, void *out, uint32_t *words
     a.index = scatter;
     a.index_count = policy->indices_count[0];
     a.rows = rows;
-    if (wire_native(a, size) && bytes <= kDirectBytes) {
+    if (wire_native(a, size) && (bytes <= kDirectBytes || in->ngroups == 1)) {
       dim3 block(128), grid(grid_for(count, 128), in->ngroups);
       bool vec = (in->nlimbs % 4 == 0) && ((uintptr_t)dst % 16 == 0);
       interleaved_to_compact<<<grid, block, 0, handle->stream>>>(in->limbs, in->nlimbs, in->stride, (uint32_t *)dst,
