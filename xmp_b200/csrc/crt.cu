@@ -38,8 +38,10 @@ XMPB_REGISTER_CRT(8, 4)
 XMPB_REGISTER_CRT(2, 24)
 XMPB_REGISTER_CRT(4, 12)
 XMPB_REGISTER_CRT(8, 6)
+XMPB_REGISTER_CRT(16, 3)
 XMPB_REGISTER_CRT(4, 16)
 XMPB_REGISTER_CRT(8, 8)
+XMPB_REGISTER_CRT(16, 4)
 XMPB_REGISTER_CRT(4, 24)
 XMPB_REGISTER_CRT(8, 12)
 XMPB_REGISTER_CRT(16, 6)

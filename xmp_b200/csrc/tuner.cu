@@ -115,10 +115,30 @@ bool tuner_lookup_powm(xmpHandle_t h, uint32_t nlimbs, uint32_t exp_bits, uint32
   int slot = tuner_lookup(h, xmpTunePowm, nlimbs * 32, exp_bits, count, &src);
   if (slot < 0 || !powm_candidate(nlimbs, slot, cfg)) return false;
   if (src == 2) {
+    // A cell of the table stands for all counts between two powers of two, by their middle, and the number of
+    // warps on the fullest scheduler steps inside it.  So the next cells' kernels are asked too, and the one that
+    // the cost model puts 8% or more below the cell's own is taken (smaller differences are the network's to
+    // judge).  Mean regret on the 409 measured powm shapes 1.01 -> 0.76%; 3072 bits x 2,001: 28.1 ms on the
+    // cell's 16 lanes, 25 on 8; 512 bits x 4,283: 677 us on one lane, 624 on 4.
+    if (cfg->dist == kDistLanes) {
+      double best = powm_shape_cycles(cfg->tpi, cfg->limbs, count, h->sm_count) / 1.08;
+      const int log2_count = 31 - __builtin_clz(count ? count : 1);
+      for (int b : {log2_count - 1, log2_count + 1}) {
+        if (b < 0 || b > 30) continue;
+        int s2 = 0;
+        PowmConfig c;
+        const int next = tuner_lookup(h, xmpTunePowm, nlimbs * 32, exp_bits, 1u << b, &s2);
+        if (next < 0 || s2 != 2 || !powm_candidate(nlimbs, next, &c) || c.dist != kDistLanes) continue;
+        const double t = powm_shape_cycles(c.tpi, c.limbs, count, h->sm_count);
+        if (t >= best) continue;
+        best = t;
+        *cfg = c;
+      }
+    }
     // The selector's window, kept within one of the analytic rule's (the network has seen exponents of
     // 17, 256, 1024 bits and the full precisions; the bound keeps it from straying elsewhere); the rule
     // alone where it wants a window beyond the six the tuner times.  On the committed B200 dataset this
-    // lowers the mean regret on all 351 powm shapes from 0.85% to 0.63% (held-out ones 1.10 -> 1.03%).
+    // lowers the mean regret on all 409 powm shapes from 0.87% to 0.58% (held-out ones 1.51 -> 1.41%).
     const int wa = window_for_bits(exp_bits, cfg->dist != kDistDigit && powm_sliding(cfg->tpi, cfg->limbs));
     cfg->window = wa > 6 ? wa : std::max(wa - 1, std::min(wa + 1, cfg->window));
   }
