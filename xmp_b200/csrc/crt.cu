@@ -13,13 +13,14 @@ std::vector<CrtKernelEntry> &crt_registry() {
   return r;
 }
 
-#define XMPB_REGISTER_CRT(TPI, L)                                                                 \
-  static void crt_launch_##TPI##_##L(const CrtArgs &a, int grid, int threads, cudaStream_t s) {  \
+#define XMPB_REGISTER_CRT_AS(TPI, L, D, NAME)                                                    \
+  static void crt_launch_##NAME(const CrtArgs &a, int grid, int threads, cudaStream_t s) {       \
     static bool attr = false;                                                                     \
-    powm_smem_attr(crt_kernel<TPI, L>, powm_smem_bytes(TPI, L), attr);                            \
-    crt_kernel<TPI, L><<<grid, threads, powm_smem_bytes(TPI, L), s>>>(a);                         \
+    powm_smem_attr(crt_kernel<TPI, L, D>, powm_smem_bytes(TPI, L), attr);                         \
+    crt_kernel<TPI, L, D><<<grid, threads, powm_smem_bytes(TPI, L), s>>>(a);                      \
   }                                                                                               \
-  static CrtKernelRegistrar crt_reg_##TPI##_##L(TPI, L, crt_launch_##TPI##_##L);
+  static CrtKernelRegistrar crt_reg_##NAME(TPI, L, D, crt_launch_##NAME);
+#define XMPB_REGISTER_CRT(TPI, L) XMPB_REGISTER_CRT_AS(TPI, L, powm_digits(TPI, L), TPI##_##L)
 
 // Shapes for halves of 256 to 4096 bits (RSA-512 to RSA-8192): two or more per size, from the fewest lanes
 // (digit kernels: most throughput) to the shortest latency.
@@ -38,6 +39,8 @@ XMPB_REGISTER_CRT(8, 4)
 XMPB_REGISTER_CRT(2, 24)
 XMPB_REGISTER_CRT(4, 12)
 XMPB_REGISTER_CRT(8, 6)
+// limbs too: a lone row of six is 10% shorter than four digits' (3072-bit keys, 593 to 1,184 at once, 5.05 / 5.72 ms)
+XMPB_REGISTER_CRT_AS(8, 6, 0, 8_6_limbs)
 XMPB_REGISTER_CRT(16, 3)
 XMPB_REGISTER_CRT(4, 16)
 XMPB_REGISTER_CRT(8, 8)
@@ -54,11 +57,12 @@ CrtConfig crt_config(uint32_t nlimbs, uint32_t exp_bits, uint32_t count, uint32_
   double best_score = 1e300;
   for (const auto &e : crt_registry()) {
     if ((uint32_t)(e.tpi * e.limbs) < nlimbs) continue;
-    const double score = powm_shape_cycles(e.tpi, e.limbs, 2.0 * count, sm_count);
+    const double score = powm_shape_cycles(e.tpi, e.limbs, 2.0 * count, sm_count, e.digits);
     if (score < best_score) {
       best_score = score;
       best.tpi = e.tpi;
       best.limbs = e.limbs;
+      best.digits = e.digits;
       best.launch = e.launch;
     }
   }
@@ -69,13 +73,12 @@ CrtConfig crt_config(uint32_t nlimbs, uint32_t exp_bits, uint32_t count, uint32_
 size_t crt_table_bytes(const CrtConfig &c, uint32_t count) {
   const size_t threads =
       round_up((uint32_t)std::min<uint64_t>((uint64_t)count * c.tpi * 2, 0xffffff80ull), (uint32_t)c.threads);
-  return threads * (size_t)powm_slot_words(c.tpi, c.limbs) * crt_table_entries(c.tpi, c.limbs, (uint32_t)c.window) * 4;
+  return threads * (size_t)crt_slot_words(c.limbs, c.digits) * crt_table_entries(c.digits, (uint32_t)c.window) * 4;
 }
 
 uint32_t crt_chunk_for(const CrtConfig &c, size_t limit, uint32_t count) {
   const uint32_t per_block = c.threads / (2 * c.tpi);  // a pair of groups per instance
-  const size_t per_inst = (size_t)2 * c.tpi * powm_slot_words(c.tpi, c.limbs) *
-                          crt_table_entries(c.tpi, c.limbs, (uint32_t)c.window) * 4;
+  const size_t per_inst = (size_t)2 * c.tpi * crt_slot_words(c.limbs, c.digits) * crt_table_entries(c.digits, (uint32_t)c.window) * 4;
   const uint64_t fit = std::min<uint64_t>(limit / per_inst, (1ull << 31) / (2 * c.tpi)) / per_block * per_block;
   return fit < per_block ? 0u : (uint32_t)std::min<uint64_t>(count, fit);
 }

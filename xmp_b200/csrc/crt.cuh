@@ -33,7 +33,7 @@ struct CrtArgs {
   uint32_t start;   // first op instance of this launch
   uint32_t count;   // op instances in this launch
   uint32_t window;  // fixed-window bits W
-  uint32_t *table;  // per warp: crt_table_entries entries x 32 lanes x powm_slot_words words
+  uint32_t *table;  // per warp: crt_table_entries entries x 32 lanes x crt_slot_words words
 };
 
 // r += x over the group; returns the carry out of the top lane (same in every lane).
@@ -373,9 +373,8 @@ __device__ __forceinline__ void dig_crt_instance(const Group<TPI> &G, const CrtA
 }
 
 // Words per lane and entries of the window table (the digit form keeps R^2 in one more).
-__host__ __device__ constexpr uint32_t crt_table_entries(int TPI, int L, uint32_t W) {
-  return (1u << W) + (powm_digits(TPI, L) ? 1u : 0u);
-}
+__host__ __device__ constexpr uint32_t crt_slot_words(int L, int D) { return D ? 2 * D : L; }
+__host__ __device__ constexpr uint32_t crt_table_entries(int D, uint32_t W) { return (1u << W) + (D ? 1u : 0u); }
 
 // The two exponentiations of an instance run side by side on two adjacent
 // groups of one warp (lanes [0, TPI) of the pair work mod p, lanes
@@ -388,8 +387,9 @@ __host__ __device__ constexpr uint32_t crt_table_entries(int TPI, int L, uint32_
 // the same Garner steps on their own modulus -- the first group's are
 // h = (mp - mq mod p) * qinv mod p and m = mq + q h, which it stores; the
 // second group's mirror image is discarded.
-template <int TPI, int L>
-__global__ void __launch_bounds__(128, powm_min_blocks(TPI, L)) crt_kernel(CrtArgs a) {
+// D: the powm kernels' digits, or 0 for limbs.
+template <int TPI, int L, int D>
+__global__ void __launch_bounds__(128, D ? powm_min_blocks(TPI, L) : 1) crt_kernel(CrtArgs a) {
   static_assert(TPI <= 16, "both groups of a pair sit in one warp");
   const DigSmem sm = powm_smem_setup<TPI, L>();
   Group<TPI> G;
@@ -399,10 +399,9 @@ __global__ void __launch_bounds__(128, powm_min_blocks(TPI, L)) crt_kernel(CrtAr
   const bool valid = local < a.count;
   // pairs past the end run a copy of the last instance so every shuffle sees a full warp
   const uint32_t i = a.start + (valid ? local : a.count - 1);
-  uint32_t *table = a.table + (size_t)(gtid >> 5) * ((size_t)32 * powm_slot_words(TPI, L) *
-                                                     crt_table_entries(TPI, L, a.window));
-  if constexpr (powm_digits(TPI, L) > 0) {
-    dig_crt_instance<TPI, L, powm_digits(TPI, L)>(G, a, i, valid, second, reinterpret_cast<double *>(table), sm);
+  uint32_t *table = a.table + (size_t)(gtid >> 5) * ((size_t)32 * crt_slot_words(L, D) * crt_table_entries(D, a.window));
+  if constexpr (D > 0) {
+    dig_crt_instance<TPI, L, D>(G, a, i, valid, second, reinterpret_cast<double *>(table), sm);
     return;
   } else {
   uint32_t *const slot = table + (size_t)(threadIdx.x & 31) * L;

@@ -12,17 +12,20 @@ typedef void (*CrtLauncher)(const CrtArgs &args, int grid, int threads, cudaStre
 struct CrtKernelEntry {
   int tpi;
   int limbs;
+  int digits;  // 52-bit digits a lane, 0: limbs
   CrtLauncher launch;
 };
 
 std::vector<CrtKernelEntry> &crt_registry();
 
 struct CrtKernelRegistrar {
-  CrtKernelRegistrar(int tpi, int limbs, CrtLauncher l) { crt_registry().push_back(CrtKernelEntry{tpi, limbs, l}); }
+  CrtKernelRegistrar(int tpi, int limbs, int digits, CrtLauncher l) {
+    crt_registry().push_back(CrtKernelEntry{tpi, limbs, digits, l});
+  }
 };
 
 struct CrtConfig {
-  int tpi = 0, limbs = 0, window = 0;
+  int tpi = 0, limbs = 0, digits = 0, window = 0;
   int threads = 128;             // per CTA; 32 where the scratch limit holds no more window tables
   CrtLauncher launch = nullptr;  // null: no kernel holds the precision
 };

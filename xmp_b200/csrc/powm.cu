@@ -67,24 +67,23 @@ bool powm_cta_preferred(uint32_t nlimbs, uint32_t count, uint32_t sm_count) {
 // (512-bit exponents; one instance, and 151,552 / TPI): a digit row of D digits takes max(155 + 8 D, 21.5 D)
 // cycles alone and 38 + 17.5 D of a full scheduler (measured / fitted: D = 5 133 / 126, 8 178 / 178, 10 212 / 213, 15
 // 293 / 301, 20 396 / 388; alone D = 4 184 / 187, 5 195 / 195, 8 215 / 219, 10 237 / 235, 15 314 / 322, 20 434 / 430); a limb
-// row max(100, 24 L) and 10 + 13.5 L (L = 4 68 / 64, 2 42 / 37; alone 32 x 2 100, 8 x 4 103).
-PowmShapeCost powm_shape_cost(int tpi, int limbs) {
-  const int d = powm_digits(tpi, limbs);
+// row max(100, 80 + 5 L) and 10 + 13.5 L (L = 6 92 / 91, 4 68 / 64, 2 42 / 37; alone L = 6 110 / 110, 4 103, 2 100).
+PowmShapeCost powm_shape_cost(int tpi, int limbs, int d) {
   const double rows = d ? (double)tpi * d : (double)tpi * limbs;
-  const double alone = d ? std::max(155.0 + 8.0 * d, 21.5 * d) : std::max(100.0, 24.0 * limbs);
+  const double alone = d ? std::max(155.0 + 8.0 * d, 21.5 * d) : std::max(100.0, 80.0 + 5.0 * limbs);
   const double full = d ? 38.0 + 17.5 * d : 10.0 + 13.5 * limbs;
   return PowmShapeCost{rows * alone, rows * full * tpi / 32.0};
 }
 
 // Two or three warps on a scheduler do not fill each other's gaps: 30 or, with the limb rows' carry chains, 35
 // cycles a row more (measured / with them, two warps: 16 x 3 133 / 136, 16 x 6 245 / 246, 8 x 12 370 / 386).
-double powm_shape_cycles(int tpi, int limbs, double groups, uint32_t sm_count) {
-  const PowmShapeCost c = powm_shape_cost(tpi, limbs);
+double powm_shape_cycles(int tpi, int limbs, double groups, uint32_t sm_count, int digits) {
+  const int d = digits < 0 ? powm_digits(tpi, limbs) : digits;
+  const PowmShapeCost c = powm_shape_cost(tpi, limbs, d);
   double warps = groups * tpi / 32.0 / (4.0 * sm_count);  // a scheduler's, four a SM
   double gaps = 0;
   if (warps < 4.0) {
     warps = ceil(warps);  // the fullest scheduler sets the time
-    const int d = powm_digits(tpi, limbs);
     if (warps > 1.0 && warps < 4.0) gaps = tpi * (d ? 30.0 * d : 35.0 * limbs);
   }
   return std::max(c.latency, c.work * 32.0 / tpi * warps + gaps);

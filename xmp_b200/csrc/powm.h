@@ -104,9 +104,10 @@ bool powm_config_valid(const PowmConfig &c, uint32_t nlimbs);
 struct PowmShapeCost {
   double latency, work;
 };
-PowmShapeCost powm_shape_cost(int tpi, int limbs);
+PowmShapeCost powm_shape_cost(int tpi, int limbs, int digits);
 // Expected cycles of a product step of `groups` lane groups on an otherwise idle GPU.
-double powm_shape_cycles(int tpi, int limbs, double groups, uint32_t sm_count);
+// (`digits`: the shape's kernel if it is not the powm one, 0 for limbs.)
+double powm_shape_cycles(int tpi, int limbs, double groups, uint32_t sm_count, int digits = -1);
 
 // Runs out = base^exp mod mod for `count` op instances starting at 0 with the
 // given configuration (validation already done).  Chunks the launch so the
