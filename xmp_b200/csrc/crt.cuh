@@ -379,7 +379,7 @@ __host__ __device__ constexpr uint32_t crt_table_entries(int D, uint32_t W) { re
 // The two exponentiations of an instance run side by side on two adjacent
 // groups of one warp (lanes [0, TPI) of the pair work mod p, lanes
 // [TPI, 2 TPI) mod q), so a batch has twice as many independent groups as
-// instances and each group does one exponentiation: measured on B200 at
+// instances and each group does one exponentiation: measured on limbs at
 // 16,384 RSA-2048 operations (4 lanes x 8 limbs), 17.8 ms against 21.6 ms
 // with both exponentiations on one group in turn, and at 1,024 operations
 // (8 x 4) 2.0 ms against 4.1 ms.  The results meet with one shuffle per limb
