@@ -234,7 +234,7 @@ static void choose_configs(xmpServer_t s, Class &c) {
     c.cfg[b] = cfg;
     c.entry[b] = powm_find(cfg.tpi, cfg.limbs);
     // small waves on a quiet GPU: one op per CTA (its constant-schedule form), at a lone op's lowest
-    // latency (one op: 3.6 vs 8.4 ms at 2048 bits, 9.2 vs 15.7 ms at 3072, 20.4 vs 30.0 ms at 4096)
+    // latency (one op: 2.9 vs 8.2 ms at 2048 bits, 6.5 vs 15.5 ms at 3072, 10.4 vs 29.3 ms at 4096)
     c.cta_limbs = powm_cta_limbs(c.n);
     c.cta[b] = c.cta_limbs != 0 && ops <= s->h->sm_count && powm_cta_preferred(c.n, ops, s->h->sm_count);
     // the kernel's Montgomery radix: limb and digit kernels of one capacity differ in it
