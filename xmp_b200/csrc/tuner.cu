@@ -117,8 +117,8 @@ bool tuner_lookup_powm(xmpHandle_t h, uint32_t nlimbs, uint32_t exp_bits, uint32
   if (src == 2) {
     // A cell of the table stands for all counts between two powers of two, by their middle, and the number of
     // warps on the fullest scheduler steps inside it.  So the next cells' kernels are asked too, and the one that
-    // the cost model puts 8% or more below the cell's own is taken (smaller differences are the network's to
-    // judge).  Mean regret on the 409 measured powm shapes 1.01 -> 0.76%; 3072 bits x 2,001: 28.1 ms on the
+    // the cost model puts 8% or more below the cell's own is taken (smaller differences are left to the
+    // network).  Mean regret on the 409 measured powm shapes 1.01 -> 0.76%; 3072 bits x 2,001: 28.1 ms on the
     // cell's 16 lanes, 25 on 8; 512 bits x 4,283: 677 us on one lane, 624 on 4.
     if (cfg->dist == kDistLanes) {
       double best = powm_shape_cycles(cfg->tpi, cfg->limbs, count, h->sm_count) / 1.08;
