@@ -380,9 +380,9 @@ template <int TPI, int L>
 __global__ void __launch_bounds__(256) divmod_lanes_kernel(DivArgs d) {
   constexpr int N = TPI * L;
   Group<TPI> G;
-  const uint32_t local = (blockIdx.x * blockDim.x + threadIdx.x) / TPI;
+  const uint64_t local = lane_instance<TPI>(blockIdx.x, blockDim.x, threadIdx.x);
   const bool valid = local < d.count;
-  const uint32_t i = valid ? local : d.count - 1;
+  const uint32_t i = valid ? (uint32_t)local : d.count - 1;
   const uint32_t ea = in_element(d.a, i), eb = in_element(d.b, i);
   const uint32_t eqo = d.q.limbs ? out_element(d.q, i) : 0, ero = d.r.limbs ? out_element(d.r, i) : 0;
   const bool store = valid && !(d.q.limbs && eqo >= d.q.count) && !(d.r.limbs && ero >= d.r.count);

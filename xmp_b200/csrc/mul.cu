@@ -129,10 +129,10 @@ template <int TPI, int L>
 __global__ void __launch_bounds__(256) mul_lanes_kernel(ArrayView a, ArrayView b, OutView c, uint32_t count) {
   static_assert(L % 4 == 0, "whole limb groups");
   Group<TPI> G;
-  const uint32_t local = (blockIdx.x * blockDim.x + threadIdx.x) / TPI;
+  const uint64_t local = lane_instance<TPI>(blockIdx.x, blockDim.x, threadIdx.x);
   const bool valid = local < count;
   // lanes past the end run a copy of the last instance so every shuffle sees a full warp
-  const uint32_t i = valid ? local : count - 1;
+  const uint32_t i = valid ? (uint32_t)local : count - 1;
   const uint32_t ea = in_element(a, i), eb = in_element(b, i), ec = out_element(c, i);
   const bool store = valid && ec < c.count;
   uint32_t A[L], r[L], c0 = 0, c1 = 0;
