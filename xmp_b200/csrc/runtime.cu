@@ -356,8 +356,9 @@ __global__ void interleaved_to_compact(const uint32_t *__restrict__ limbs, uint3
 }
 
 // A few native rows passed by value: a synchronous import of pageable rows up to kSmallImportBytes needs no
-// copy in front of its kernel (256-bit rows x 100, two imports, an add and an export: 59 -> 52 us together
-// with the export's mailbox).  The kernel's parameters are 4 KB; larger rows gain nothing from it.
+// copy in front of its kernel (256-bit rows x 100, two imports, an add and an export: 59.2 -> 55.8 us together
+// with the export's mailbox, timed in turn on one machine; 61.1 -> 57.6 on another).  The limit leaves the
+// parameters inside the 4 KB that every launch path takes; larger ones were not timed.
 struct SmallRows {
   uint32_t w[kSmallImportBytes / 4];
 };
@@ -673,16 +674,19 @@ static xmpError_t import_internal(xmpHandle_t handle, xmpIntegers_t out, uint32_
   const void *src = in;
   bool pageable = false;
   if (is_host_pointer(in, &pageable)) {
+    // The arena first in every case: a caller warms up with the plain form before it captures the asynchronous one.
+    xmpError_t e = ensure_scratch(handle, bytes);
+    if (e != xmpErrorSuccess) return e;
     // Only where the host may read the rows now: the asynchronous form may be captured and replayed, pinned
     // rows may be the target of a copy of any stream, and work on this one may yet write pageable rows.
     bool now = !async && pageable && bytes <= kSmallImportBytes && size == 4 && order == -1 &&
                endian == native_endian() && nails == 0 && gather == nullptr;
-    if (now && cudaStreamQuery(handle->stream) != cudaSuccess) {
-      cudaGetLastError();
-      now = false;
+    if (now) {
+      const cudaError_t idle = cudaStreamQuery(handle->stream);
+      if (idle == cudaErrorNotReady) cudaGetLastError();
+      now = idle == cudaSuccess;
     }
     if (now) {
-      if (bytes > scratch_limit(handle)) return xmpErrorIncreaseScratchLimit;  // as the staged copy below
       SmallRows r;
       memcpy(r.w, in, bytes);
       small_rows_to_interleaved<<<dim3(grid_for(count, 128), out->ngroups), 128, 0, handle->stream>>>(
@@ -691,8 +695,6 @@ static xmpError_t import_internal(xmpHandle_t handle, xmpIntegers_t out, uint32_
       return check_cuda();
     }
     rows = count;
-    xmpError_t e = ensure_scratch(handle, bytes);
-    if (e != xmpErrorSuccess) return e;
     if (cudaMemcpyAsync(handle->scratch, in, bytes, cudaMemcpyHostToDevice, handle->stream) != cudaSuccess)
       return xmpErrorCuda;
     src = handle->scratch;
@@ -757,15 +759,11 @@ static xmpError_t export_internal(xmpHandle_t handle, void *out, uint32_t *words
   // the wait (other formats leave in pieces too small for the bus).
   const bool mail = host && !async && pageable && handle->mailbox && bytes <= kMailboxBytes && scatter == nullptr &&
                     size == 4 && order == -1 && endian == native_endian() && nails == 0;
-  if (mail) {
-    if (bytes > scratch_limit(handle)) return xmpErrorIncreaseScratchLimit;  // as the staged copy
+  if (host) {
     rows = count;
-    dst = handle->mailbox;
-  } else if (host) {
-    rows = count;
-    xmpError_t e = ensure_scratch(handle, bytes);
+    xmpError_t e = ensure_scratch(handle, bytes);  // taken through the mailbox or not, as an import
     if (e != xmpErrorSuccess) return e;
-    dst = handle->scratch;
+    dst = mail ? handle->mailbox : handle->scratch;
     if (scatter) {
       // Scattered rows not written by this call keep the caller's contents.
       if (cudaMemcpyAsync(dst, out, bytes, cudaMemcpyHostToDevice, handle->stream) != cudaSuccess) return xmpErrorCuda;
