@@ -281,7 +281,8 @@ xmpError_t XMPAPI xmpPowmBatchPlanCreate(xmpHandle_t h, const xmpPowmBatchItem_t
   }
   // CRT items: window tables for all instances at once, or chunks of what half the scratch limit holds
   for (auto &c : p->crt) {
-    if ((c.chunk = crt_fit(c.cfg, scratch_limit(h) / 2, c.item.count)) == 0) return fail(xmpErrorIncreaseScratchLimit);
+    c.chunk = crt_fit(c.cfg, c.item.p->nlimbs, scratch_limit(h) / 2, c.item.count);
+    if (c.chunk == 0) return fail(xmpErrorIncreaseScratchLimit);
     c.table_offset = bytes;
     bytes += crt_table_bytes(c.cfg, c.chunk);
     bytes = (bytes + 255) & ~(size_t)255;

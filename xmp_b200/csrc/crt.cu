@@ -83,12 +83,32 @@ uint32_t crt_chunk_for(const CrtConfig &c, size_t limit, uint32_t count) {
   return fit < per_block ? 0u : (uint32_t)std::min<uint64_t>(count, fit);
 }
 
-uint32_t crt_fit(CrtConfig &c, size_t limit, uint32_t count) {
+// Bytes of one warp's window-1 table, the least a shape can run with.
+static size_t crt_least_bytes(int limbs, int digits) {
+  return (size_t)32 * crt_slot_words(limbs, digits) * crt_table_entries(digits, 1) * 4;
+}
+
+uint32_t crt_fit(CrtConfig &c, uint32_t nlimbs, size_t limit, uint32_t count) {
   uint32_t chunk;
   while ((chunk = crt_chunk_for(c, limit, count)) == 0) {
-    if (c.window > 1) c.window--;
-    else if (c.threads > 32) c.threads = 32;
-    else return 0;
+    if (c.window > 1) {
+      c.window--;
+    } else if (c.threads > 32) {
+      c.threads = 32;
+    } else {
+      // The shape was chosen for its speed (one lane of 20 digits takes 15 KB); the limit decides before that.
+      const size_t least = crt_least_bytes(c.limbs, c.digits);
+      size_t best = least;
+      for (const auto &e : crt_registry()) {
+        if ((uint32_t)(e.tpi * e.limbs) < nlimbs || crt_least_bytes(e.limbs, e.digits) >= best) continue;
+        best = crt_least_bytes(e.limbs, e.digits);
+        c.tpi = e.tpi;
+        c.limbs = e.limbs;
+        c.digits = e.digits;
+        c.launch = e.launch;
+      }
+      if (best == least) return 0;
+    }
   }
   return chunk;
 }
@@ -146,7 +166,7 @@ xmpError_t XMPAPI xmpIntegersPowmCRTAsync(xmpHandle_t h, xmpIntegers_t out, cons
   CrtConfig cfg = crt_config(p->nlimbs, std::max(dp->precision, dq->precision), count, h->sm_count);
   if (!cfg.launch) return xmpErrorUnsupported;
   // chunk so the window tables fit the scratch limit; shrink the window when one block does not fit
-  const uint32_t chunk = crt_fit(cfg, scratch_limit(h), count);
+  const uint32_t chunk = crt_fit(cfg, p->nlimbs, scratch_limit(h), count);
   if (chunk == 0) return xmpErrorIncreaseScratchLimit;
   // an output that is also an input is written through the handle's temporary output buffer
   const bool aliased = (out == c || out == p || out == q || out == dp || out == dq || out == qinv);
