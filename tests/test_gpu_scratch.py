@@ -77,3 +77,27 @@ def test_crt_within_a_small_limit(bits, count, limit, plan):
         v.destroy()
     pol.destroy()
     h.destroy()
+
+
+# The limit: 128 threads' window-1 tables in limbs on the lanes of the kernel that was faster on them.
+@pytest.mark.parametrize("bits,count,limit", [(256, 128, 2048), (512, 6144, 4096), (1024, 32768, 8192),
+                                              (1536, 6144, 6144), (2048, 1536, 4096), (3072, 3072, 6144)])
+def test_powm_within_a_small_limit(bits, count, limit):
+    h = xmp.Handle()
+    r = np.random.default_rng(bits)
+    n = bits // 32
+    x, m = (r.integers(0, 1 << 32, (count, n), dtype=np.uint32) for _ in range(2))
+    e = r.integers(0, 1 << 32, (count, 1), dtype=np.uint32)
+    m[:, 0] |= 1
+    X, E, M, O = h.integers(bits, count, x), h.integers(32, count, e), h.integers(bits, count, m), h.integers(bits, count)
+    pol = h.policy()
+    pol.set_scratch_limit(limit)
+    h.set_policy(pol)
+    xmp.powm(h, O, X, E, M, count)
+    h.set_policy(None)
+    want = [pow(a, b, c) for a, b, c in zip(*(ints_from_rows(v) for v in (x, e, m)))]
+    assert ints_from_rows(O.export()) == want
+    for v in (X, E, M, O):
+        v.destroy()
+    pol.destroy()
+    h.destroy()

@@ -208,6 +208,23 @@ xmpError_t powm_run(xmpHandle_t h, const PowmConfig &cfg0, const OutView &out, c
 
 }  // namespace xmpb
 
+// Bytes of one warp's window-1 table, the least a lane kernel can run with.
+static size_t powm_least_bytes(int tpi, int limbs) {
+  return (size_t)32 * powm_slot_words(tpi, limbs) * powm_table_entries(1, powm_sliding(tpi, limbs)) * 4;
+}
+
+// Kernels chosen for their speed alone keep up to 20 digits a lane, 10 KB for one warp; where the scratch limit
+// is below that, the kernel with the smallest tables that holds the precision takes their place.
+static void powm_within_limit(PowmConfig &cfg, uint32_t nlimbs, size_t limit) {
+  if (cfg.dist != kDistLanes || powm_least_bytes(cfg.tpi, cfg.limbs) <= limit) return;
+  for (const auto &e : powm_registry()) {
+    if ((uint32_t)(e.tpi * e.limbs) < nlimbs) continue;
+    if (powm_least_bytes(e.tpi, e.limbs) >= powm_least_bytes(cfg.tpi, cfg.limbs)) continue;
+    cfg.tpi = e.tpi;
+    cfg.limbs = e.limbs;
+  }
+}
+
 // The configuration for a problem shape under the handle's policy (default algorithm): a choice set
 // for the exact shape, else one instance per CTA for small batches, else the selector, else the
 // heuristic.  An explicit algorithm takes the heuristic restricted to it.
@@ -225,6 +242,7 @@ static PowmConfig powm_choose_config(xmpHandle_t h, uint32_t nlimbs, uint32_t ex
     return cfg;
   }
   if (!tuned) cfg = powm_default_config(nlimbs, exp_bits, count, alg, h->sm_count);
+  if (alg == xmpAlgorithmDefault) powm_within_limit(cfg, nlimbs, scratch_limit(h));
   return cfg;
 }
 
