@@ -581,10 +581,23 @@ xmpError_t XMPAPI xmpServerCreate(xmpHandle_t h, const uint32_t *precisions, uin
       if (!c.entry[b]) return fail(xmpErrorUnsupported);
     c.kcap = round_up(cf.max_keys, 32);
   }
-  // Equal slot counts per class, within the budget.  A budget too small for one granule of slots takes
-  // smaller windows, then one Montgomery radix per class (the first bucket's kernel for every wave).
+  // Equal slot counts per class, within the budget.  At least as many, up to a full wave's, as window tables in
+  // limbs and one R^2 per key would leave: a digit is held in 64 bits, so its tables are up to a third larger,
+  // and the budget decides which requests are admitted (max_wave_ops operations at most).  A budget that holds
+  // fewer takes smaller windows, then one Montgomery radix per class (the first bucket's kernel for every wave).
+  uint64_t want = granule;
+  for (uint32_t i = 0; i < n_classes; i++) {
+    const Class &c = s->classes[i];
+    key_bytes += 2 * (size_t)c.ngroups * 16 * c.kcap;
+    per_slot_total += 3 * (size_t)c.ngroups * 16 + 4 + 3 * (size_t)c.n * 4 +
+                      (size_t)c.cap * powm_table_entries(c.cfg[0].window, false) * 4;
+  }
+  if (cf.hbm_budget > key_bytes) {
+    const uint64_t in_limbs = std::min<uint64_t>((cf.hbm_budget - key_bytes) / per_slot_total, cf.max_slots);
+    want = std::max(want, std::min<uint64_t>(in_limbs / granule * granule, round_up(cf.max_wave_ops, granule)));
+  }
   uint64_t slots = 0;
-  for (int step = 0; step < 14 && slots < granule; step++) {
+  for (int step = 0; step < 14 && slots < want; step++) {
     const int max_window = 7 - step % 7;
     key_bytes = per_slot_total = 0;
     for (uint32_t i = 0; i < n_classes; i++) {
