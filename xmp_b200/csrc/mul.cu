@@ -125,6 +125,19 @@ __global__ void __launch_bounds__(256) mul_reg_kernel(ArrayView a, ArrayView b, 
 // Measured (B200) against the streamed kernel below, which loads both limbs of every limb product: 2048 x
 // 2048 bits x 10,001 332 -> 21 us, 4096 x 4,096 1,174 -> 29 us, 8192 x 2,048 6,632 -> 52 us, 1536 x 32,768
 // 191 -> 27 us.
+// The product may take an operand's place (no index arrays): the larger operand is read before the first store,
+// group g of the smaller one before group g - 1 of the product is stored, by every lane (the barrier), and
+// plain loads, since the read-only path takes memory that the kernel does not write.
+__device__ __forceinline__ uint4 load_group_rw(const ArrayView &v, uint32_t e, uint32_t g) {
+  if (g * 4 >= v.nlimbs) return make_uint4(0, 0, 0, 0);
+  uint4 x = reinterpret_cast<const uint4 *>(v.limbs)[(size_t)g * v.stride + e];
+  const uint32_t rem = v.nlimbs - g * 4;
+  if (rem < 2) x.y = 0;
+  if (rem < 3) x.z = 0;
+  if (rem < 4) x.w = 0;
+  return x;
+}
+
 template <int TPI, int L>
 __global__ void __launch_bounds__(256) mul_lanes_kernel(ArrayView a, ArrayView b, OutView c, uint32_t count) {
   static_assert(L % 4 == 0, "whole limb groups");
@@ -136,17 +149,24 @@ __global__ void __launch_bounds__(256) mul_lanes_kernel(ArrayView a, ArrayView b
   const uint32_t ea = in_element(a, i), eb = in_element(b, i), ec = out_element(c, i);
   const bool store = valid && ec < c.count;
   uint32_t A[L], r[L], c0 = 0, c1 = 0;
-  load_lane_limbs<TPI, L>(A, a.limbs, a.nlimbs, a.stride, ea, G.lane);
+#pragma unroll
+  for (int m = 0; m < L / 4; m++) {
+    const uint4 v = load_group_rw(a, ea, G.lane * (L / 4) + m);
+    A[4 * m] = v.x;
+    A[4 * m + 1] = v.y;
+    A[4 * m + 2] = v.z;
+    A[4 * m + 3] = v.w;
+  }
 #pragma unroll
   for (int k = 0; k < L; k++) r[k] = 0;
   uint32_t base = 0;
-  uint4 w4 = load_group(b.limbs, b.nlimbs, b.stride, eb, 0);
+  uint4 w4 = load_group_rw(b, eb, 0);
 #pragma unroll 1
   for (; base < b.nlimbs; base += L) {
 #pragma unroll
     for (int m = 0; m < L / 4; m++) {
       const uint32_t w[4] = {w4.x, w4.y, w4.z, w4.w};
-      w4 = load_group(b.limbs, b.nlimbs, b.stride, eb, base / 4 + m + 1);
+      w4 = load_group_rw(b, eb, base / 4 + m + 1);
       uint32_t done[4];
 #pragma unroll
       for (int t = 0; t < 4; t++) {
@@ -162,6 +182,7 @@ __global__ void __launch_bounds__(256) mul_lanes_kernel(ArrayView a, ArrayView b
         c0 = addc_fma(c1);
         c1 = 0;
       }
+      __syncwarp();
       if (G.lane == 0 && store && base + 4 * m < c.nlimbs)
         store_group(c.limbs, c.nlimbs, c.stride, ec, base / 4 + m, make_uint4(done[0], done[1], done[2], done[3]));
     }
@@ -303,7 +324,8 @@ xmpError_t mul_entry(xmpHandle_t h, xmpIntegers_t p, xmpIntegers_t a, xmpInteger
   bool aliased = (p == a || p == b);
   bool indexed = pol->indices[0] || pol->indices[1] || pol->indices[2];
   OutTarget t;
-  // The streamed kernel reads inputs while writing the product: stage whenever it aliases.
+  // The streamed kernel reads inputs while writing the product: stage whenever it aliases.  The register and lane
+  // kernels read an instance's limbs before they overwrite them: stage only where an index may move instances.
   xmpError_t e = begin_output(h, p, aliased, indexed || !launch, &t);
   if (e != xmpErrorSuccess) return e;
   OutView vc = view_out(p, t.limbs, pol->indices[0]);
