@@ -117,8 +117,8 @@ xmpError_t XMPAPI xmpPowmBatchPlanInfo(xmpPowmBatchPlan_t plan, int32_t *bins, u
  *   powm:   slot = 6*d + (W-1), d in {per-thread, 2, 4, 8, 16, 32 lanes,
  *           digit-serial}, W = window bits 1..6 (42 slots; each lane count uses
  *           the fewest limbs per lane that hold the precision);
- *   mul, divmod: slot = 4*v + t, v in {register kernel, streamed kernel},
- *           t -> 32, 64, 128, 256 threads per block (8 slots).
+ *   mul, divmod: slot = 4*v + t, v in {register kernel, lane kernel (above
+ *           512 limbs: streamed)}, t -> 32, 64, 128, 256 threads per block (8 slots).
  * Slots a shape cannot use are invalid. */
 enum { xmpTuneMul = 0, xmpTuneDivMod = 1, xmpTunePowm = 2 };
 #define XMP_TUNE_CANDIDATES 48
@@ -132,7 +132,7 @@ typedef struct {
 
 /* Whether `slot` is a valid candidate for (op, bits) and the configuration it
  * stands for (powm: all four fields; mul/divmod: distribution = 0 register /
- * 1 streamed, lanes = threads per block). */
+ * 1 lane or streamed kernel, lanes = threads per block). */
 xmpError_t XMPAPI xmpTuneCandidate(int32_t op, uint32_t bits, int32_t slot, int32_t *valid,
                                    xmpPowmConfig_t *config);
 
@@ -148,7 +148,12 @@ xmpError_t XMPAPI xmpTuneMeasure(xmpHandle_t handle, const xmpTuneShape_t *shape
  * built-in heuristic (source 1, 2, 0).  A new handle starts with the
  * selector compiled into the library (trained on this library's B200
  * timings) loaded; xmpTuneClear drops every choice and the selector, leaving
- * the heuristic. */
+ * the heuristic.  A choice set for the exact shape runs as it is.  From the
+ * selector xmpTuneGetChoice returns the table's cell, which stands for a range
+ * of counts: powm may run the kernel of a neighbouring range of counts where
+ * the library's cost model puts that one clearly lower for this count, its
+ * window follows the exponent length, small batches run one instance per CTA
+ * and divmod may take the lane kernel.  xmpPowmGetConfig says what a powm runs. */
 xmpError_t XMPAPI xmpTuneSetChoice(xmpHandle_t handle, const xmpTuneShape_t *shape, int32_t slot);
 xmpError_t XMPAPI xmpTuneGetChoice(xmpHandle_t handle, const xmpTuneShape_t *shape, int32_t *slot, int32_t *source);
 xmpError_t XMPAPI xmpTuneClear(xmpHandle_t handle);

@@ -15,8 +15,6 @@ std::vector<CrtKernelEntry> &crt_registry() {
 
 #define XMPB_REGISTER_CRT_AS(TPI, L, D, NAME)                                                    \
   static void crt_launch_##NAME(const CrtArgs &a, int grid, int threads, cudaStream_t s) {       \
-    static bool attr = false;                                                                     \
-    powm_smem_attr(crt_kernel<TPI, L, D>, powm_smem_bytes(TPI, L), attr);                         \
     crt_kernel<TPI, L, D><<<grid, threads, powm_smem_bytes(TPI, L), s>>>(a);                      \
   }                                                                                               \
   static CrtKernelRegistrar crt_reg_##NAME(TPI, L, D, crt_launch_##NAME);

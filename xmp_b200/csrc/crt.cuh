@@ -387,7 +387,9 @@ __host__ __device__ constexpr uint32_t crt_table_entries(int D, uint32_t W) { re
 // the same Garner steps on their own modulus -- the first group's are
 // h = (mp - mq mod p) * qinv mod p and m = mq + q h, which it stores; the
 // second group's mirror image is discarded.
-// D: the powm kernels' digits, or 0 for limbs.
+// D: the powm kernels' digits, or 0 for limbs, with their bound on CTAs per SM, at which this kernel's longer
+// state spills up to 208 bytes a thread.  With one CTA fewer (two at least) RSA-4096 x 2,048 takes 11.3 ms
+// instead of 12.3, RSA-2048 x 4,096 3.13 instead of 3.37, x 16,384 10.9 instead of 10.8: the bound was not fitted here.
 template <int TPI, int L, int D>
 __global__ void __launch_bounds__(128, D ? powm_min_blocks(TPI, L) : 1) crt_kernel(CrtArgs a) {
   static_assert(TPI <= 16, "both groups of a pair sit in one warp");

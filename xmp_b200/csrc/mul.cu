@@ -287,8 +287,9 @@ bool mul_has_register_kernel(uint32_t na, uint32_t nb) {
   return al && bl && pick_mul(al, bl) != nullptr;
 }
 
-// Register kernel when one exists for the operand classes (else the streamed
-// kernel), 128 threads -- unless the tuner or the caller chose otherwise.
+// Register kernel when one exists for the operand classes, else the lane kernel
+// up to 512 limbs, else the streamed one; 128 threads -- unless the tuner or the
+// caller chose otherwise (an explicit digit-serial algorithm is streamed).
 xmpError_t mul_entry(xmpHandle_t h, xmpIntegers_t p, xmpIntegers_t a, xmpIntegers_t b, uint32_t count,
                      const ElemConfig *forced) {
   if (!h || !p || !a || !b) return xmpErrorInvalidParameter;

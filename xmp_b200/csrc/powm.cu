@@ -46,8 +46,8 @@ int window_for_bits(uint32_t exp_bits, bool sliding) {
 bool powm_cta_preferred(uint32_t nlimbs, uint32_t count, uint32_t sm_count) {
   const uint32_t limbs = powm_cta_limbs(nlimbs);
   // Up to 512 bits the smallest CTA (1024-bit operands) pads too much: it ties with the lane kernels at 512
-  // bits (0.55 ms for 148 instances, 0.59 ms for 296, vs 0.59 ms) and loses below (384 bits 0.44 ms vs 0.48 on 8
-  // lanes, less on fewer).  From 544 bits on it is faster alone at every measured size (544: 0.57 vs 1.11 ms on 8 x 4,
+  // bits (0.55 ms for 148 instances, 0.59 ms for 296, vs 0.59 ms on 4 x 4) and loses below (148 instances of 384
+  // bits 0.43 ms vs 0.33 on 4 x 3, 256 bits 0.32 vs 0.15 on 1 x 8).  From 544 bits on it is faster alone at every measured size (544: 0.57 vs 1.11 ms on 8 x 4,
   // 1056: 1.40 vs 2.86, 1536: 1.97 vs 4.04, 2048: 2.56 vs 7.6, 3072: 5.94 vs 15.6, 4096: 9.7 vs 29.3 ms).
   if (!limbs || nlimbs <= 16) return false;
   // A CTA per instance runs it near its lone latency while the SMs hold the batch; the lane kernels
@@ -55,8 +55,8 @@ bool powm_cta_preferred(uint32_t nlimbs, uint32_t count, uint32_t sm_count) {
   // exponents), CTA at 148 / 296 / 444 / 592 / 888 instances vs the best lane kernel: 768 bits
   // 0.78/0.84/0.91/0.97/1.20 vs 1.11 ms; 1024 bits 0.99/1.07/1.17/1.25/1.54 vs 2.03 ms; 1536 bits
   // 1.98/2.51/4.35 vs 4.03 ms; 2048 bits 2.58/3.27/5.68/6.52 vs 7.7 ms; 3072 bits 5.98/11.9 vs 15.6 ms;
-  // 4096 bits 9.8/19.5 vs 29.5 ms.  The limits are the ones that callers of the default have had: above
-  // 1024 bits a second or fourth CTA per SM would gain as well.
+  // 4096 bits 9.8/19.5 vs 29.5 ms.  The limits are older than these times and not fitted to them: above 2048 bits
+  // two CTAs per SM and at 2048 bits four would gain as well.
   uint32_t per_sm = 1;
   if (limbs == 32) per_sm = nlimbs > 24 ? 6 : 4;
   else if (limbs == 64) per_sm = nlimbs > 48 ? 3 : 2;
@@ -105,7 +105,8 @@ PowmConfig powm_default_config(uint32_t nlimbs, uint32_t exp_bits, uint32_t coun
     best.dist = kDistDigit;
     return best;
   }
-  // Enough lanes to give every SM a few warps; below that, spread instances wider.
+  // A score in limb multiply-adds, fitted before the digit kernels (powm_shape_cycles is their model).  Enough lanes
+  // to give every SM a few warps; below that, spread instances wider.
   const double want_threads = (double)sm_count * 4 * 32;
   double best_score = 1e300;
   for (const auto &e : powm_registry()) {

@@ -50,32 +50,18 @@ struct PowmKernelRegistrar {
   }
 };
 
-// Raises a kernel's dynamic shared memory limit above the 48 KB default once (needs a current device).
-template <class F>
-inline void powm_smem_attr(F *fn, uint32_t bytes, bool &done) {
-  if (!done && bytes > 48 * 1024) {
-    cudaFuncSetAttribute((const void *)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-    done = true;
-  }
-}
-
+// Dynamic shared memory stays below the 48 KB that every launch may ask for (20 KB at 20 digits a lane).
 #define XMPB_REGISTER_POWM(TPI, L)                                                                       \
   static void powm_launch_##TPI##_##L(const PowmArgs &a, int grid, int threads, cudaStream_t s) {        \
-    static bool attr = false;                                                                            \
-    powm_smem_attr(powm_kernel<TPI, L>, powm_smem_bytes(TPI, L), attr);                                  \
     powm_kernel<TPI, L><<<grid, threads, powm_smem_bytes(TPI, L), s>>>(a);                               \
   }                                                                                                      \
   static void powm_launch_batch_##TPI##_##L(const PowmBatchArgs &a, int grid, cudaStream_t s) {          \
-    static bool attr = false;                                                                            \
-    powm_smem_attr(powm_batch_kernel<TPI, L>, powm_smem_bytes(TPI, L), attr);                            \
     powm_batch_kernel<TPI, L><<<grid, 128, powm_smem_bytes(TPI, L), s>>>(a);                             \
   }                                                                                                      \
   static void powm_launch_r2_##TPI##_##L(const PowmArgs &a, int grid, int threads, cudaStream_t s) {     \
     r2_kernel<TPI, L><<<grid, threads, powm_smem_bytes(TPI, L), s>>>(a);                                 \
   }                                                                                                      \
   static void powm_launch_ct_##TPI##_##L(const PowmArgs &a, int grid, int threads, cudaStream_t s) {     \
-    static bool attr = false;                                                                            \
-    powm_smem_attr(powm_kernel<TPI, L, true>, powm_smem_bytes(TPI, L), attr);                            \
     powm_kernel<TPI, L, true><<<grid, threads, powm_smem_bytes(TPI, L), s>>>(a);                         \
   }                                                                                                      \
   static PowmKernelRegistrar powm_reg_##TPI##_##L(TPI, L, powm_launch_##TPI##_##L,                       \
@@ -93,8 +79,8 @@ inline void powm_smem_attr(F *fn, uint32_t bytes, bool &done) {
 int window_for_bits(uint32_t exp_bits, bool sliding = true);
 
 // Heuristic configuration for n-limb moduli (used when no tuned entry exists).
-// A nonzero `cap` admits only kernels with exactly cap = lanes x limbs (the
-// Montgomery radix R = 2^(32 cap) of precomputed constants).
+// Scores limb multiply-adds (powm.cu).  A nonzero `cap` admits only kernels with
+// exactly cap = lanes x limbs (whose Montgomery radices differ: powm_radix_bits).
 PowmConfig powm_default_config(uint32_t nlimbs, uint32_t exp_bits, uint32_t count, xmpAlgorithm_t alg,
                                uint32_t sm_count, uint32_t cap = 0);
 bool powm_config_valid(const PowmConfig &c, uint32_t nlimbs);

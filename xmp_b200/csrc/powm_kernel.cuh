@@ -8,10 +8,12 @@
 // kernel (powm_implementations.h:122-152 / 480-516).
 //
 // Per instance:
-//   1. N, n0' = -N^-1 mod 2^32, R^2 mod N (exact doublings + Montgomery squarings)
-//   2. window table, stored in the scratch arena, one contiguous slot of L
-//      limbs per lane so every lane moves its limbs with 128-bit accesses:
-//      slot 0 = R - N (Mont(1)), then for the sliding window the odd powers
+//   1. N, -N^-1 mod 2^32 (mod 2^52 on digits), R^2 mod N (exact doublings +
+//      Montgomery squarings), in the shape's arithmetic: 32-bit limbs (mont.cuh)
+//      below six a lane, 52-bit digits (dmont.cuh) from there on (powm_digits)
+//   2. window table, stored in the scratch arena (limbs: one contiguous slot of
+//      L limbs per lane, moved with 128-bit accesses; digits: dig_slot_store):
+//      slot 0 = Mont(1), then for the sliding window the odd powers
 //      Mont(x^(2j-1)), j = 1 .. 2^(W-1) (one squaring for Mont(x^2), then one
 //      multiply per entry), for the fixed window Mont(x^e), e < 2^W
 //   3. the exponent, left to right, by the shape's method (powm_sliding):
@@ -48,7 +50,7 @@ namespace xmpb {
 struct PowmArgs {
   ArrayView base, exp, mod;
   ArrayView r2;     // optional (limbs == nullptr: computed per instance): R^2 mod N per modulus element,
-                    // R = 2^(32 * TPI * L), indexed like `mod`
+                    // R = 2^powm_radix_bits(TPI, L), indexed like `mod`
   OutView out;
   uint32_t start;   // first op instance of this launch
   uint32_t count;   // op instances in this launch
@@ -591,20 +593,12 @@ __device__ __forceinline__ void powm_instance(const Group<TPI> &G, const PowmArg
 // (8 x 12); at 5 digits 7 / 6 / 5 took 7.2 / 6.7 / 6.8 ms (4 x 8), with one
 // instance alone 15% faster at 5; at 15 digits 3 / 2 took 46.7 / 44.9 ms
 // (4 x 24) and 13.2 / 11.4 ms (1 x 24, with the square's 30 columns).
+// 20 digits on several lanes take all 255 registers and spill (stores / loads,
+// bytes a thread: 2 x 32 80 / 348, 4 x 32 80 / 352; one lane, with its own
+// square, none).
 constexpr int powm_min_blocks(int TPI, int L) {
   const int D = powm_digits(TPI, L);
   return D == 0 ? 1 : D <= 5 ? 5 : D <= 10 ? 4 : 2;
-}
-
-// Resident CTAs of 128 threads asked of the register allocator for the
-// persistent kernel: left alone, its extra loop state made the allocator take
-// ~124 registers at 10-12 limbs per lane (4 CTAs/SM) where the one-shot
-// kernel needs 96 (5 CTAs/SM).  The one-shot kernel keeps the allocator's own
-// choice (a bound equal to its natural count still changed its schedule and
-// cost 2.4% at 2048 bits).
-constexpr int powm_batch_min_blocks(int TPI, int L) {
-  if (powm_digits(TPI, L)) return powm_min_blocks(TPI, L);
-  return 1;
 }
 
 template <int TPI, int L, bool CT = false>
@@ -670,7 +664,7 @@ struct PowmBatchArgs {
 };
 
 template <int TPI, int L>
-__global__ void __launch_bounds__(128, powm_batch_min_blocks(TPI, L)) powm_batch_kernel(PowmBatchArgs b) {
+__global__ void __launch_bounds__(128, powm_min_blocks(TPI, L)) powm_batch_kernel(PowmBatchArgs b) {
   const DigSmem sm = powm_smem_setup<TPI, L>();
   Group<TPI> G;
   const uint32_t gwarp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;

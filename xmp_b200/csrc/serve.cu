@@ -219,8 +219,9 @@ static void free_all(xmpServer_t s) {
 }
 
 // Configuration per wave-size bucket: the tuner's choice (an exact tuned entry
-// or the learned selector) when it runs at the class's Montgomery radix, else
-// the built-in heuristic restricted to that radix.
+// or the learned selector) when its kernel has the class's capacity (lanes x
+// limbs), else the built-in heuristic restricted to it.  Kernels of one capacity
+// differ in their Montgomery radix, limbs and digits; R^2 is kept for each.
 static void choose_configs(xmpServer_t s, Class &c) {
   c.nradix = 0;
   for (int b = 0; b < kBuckets; b++) {
@@ -556,7 +557,7 @@ xmpError_t XMPAPI xmpServerCreate(xmpHandle_t h, const uint32_t *precisions, uin
     return e;
   };
   const uint32_t granule = 128;
-  // ---- classes: radix, configurations, per-slot footprint ----
+  // ---- classes: capacity, configurations, per-slot footprint ----
   s->classes.resize(n_classes);
   size_t key_bytes = 0, per_slot_total = 0;
   std::vector<size_t> per_slot(n_classes);
@@ -568,7 +569,7 @@ xmpError_t XMPAPI xmpServerCreate(xmpHandle_t h, const uint32_t *precisions, uin
     c.precision = precisions[i];
     c.n = precisions[i] / 32;
     c.ngroups = div_up(c.n, 4);
-    // Montgomery radix: the smallest register-kernel capacity that holds n limbs
+    // the smallest register-kernel capacity that holds n limbs
     uint32_t cap = 0;
     for (const auto &e : powm_registry()) {
       uint32_t k = (uint32_t)e.tpi * e.limbs;

@@ -1,7 +1,7 @@
 // Squaring-specialised Montgomery product: r = a^2 R^-1 mod N, almost reduced
-// (r < R), for the exponentiation's squarings (the reference's per-thread
-// sqr, regmp/sqr_imad.h:25-78, used by its powm model powm/three_n.h; here
-// also for the four-lane distribution).
+// (r < R), for the exponentiation's squarings on one lane (the reference's
+// per-thread sqr, regmp/sqr_imad.h:25-78, used by its powm model
+// powm/three_n.h).
 //
 // Separated operand scanning: the square T = a^2 is formed first with each
 // cross product a_i a_j (i < j) computed once and doubled, then reduced by the
@@ -10,8 +10,8 @@
 // costs n(n+1)/2 products instead of n^2, so a Montgomery squaring costs about
 // 3n^2/2 + n products instead of 2n^2 + n.
 //
-// Per-thread (TPI = 1): T is formed in registers; the reduction takes T's low
-// half as the accumulator and shifts T's high words in at the top.
+// T is formed in registers; the reduction takes T's low half as the
+// accumulator and shifts T's high words in at the top.
 #pragma once
 #include "dmont.cuh"
 #include "mont.cuh"
@@ -56,21 +56,19 @@ __device__ __forceinline__ void lane_square(uint32_t (&s)[2 * L], const uint32_t
   }
 }
 
-// One quotient row of the reduction: acc += N q (q from the group's lowest word), then the
-// accumulator shifts down one word with `in` (a word of T, or zero) entering at the top of the top lane.
-template <int TPI, int L>
-__device__ __forceinline__ void redc_row(const Group<TPI> &G, uint32_t (&r)[L], uint32_t &c0, uint32_t &c1,
-                                         const uint32_t (&n)[L], uint32_t np0, uint32_t in) {
-  const uint32_t q = G.bcast(r[0], 0) * np0;
+// One quotient row of the reduction: acc += N q (q from the lowest word), then the accumulator shifts down one
+// word with `in` (a word of T) entering at the top.
+template <int L>
+__device__ __forceinline__ void redc_row(uint32_t (&r)[L], uint32_t &c0, uint32_t &c1, const uint32_t (&n)[L],
+                                         uint32_t np0, uint32_t in) {
+  const uint32_t q = r[0] * np0;
   uint64_t s[L];
   row_products<L>(s, n, q);
   add_low_halves<L>(r, c0, c1, s);
   add_high_halves<L>(r, c0, c1, s);
-  uint32_t t = TPI == 1 ? in : G.from_next(r[0]);
-  if (TPI > 1 && G.lane == TPI - 1) t = in;
 #pragma unroll
   for (int j = 0; j < L - 1; j++) r[j] = r[j + 1];
-  r[L - 1] = add_cc(t, c0);
+  r[L - 1] = add_cc(in, c0);
   c0 = addc_fma(c1);
   c1 = 0;
 }
@@ -85,7 +83,7 @@ __device__ __forceinline__ void mont_sqr1(const Group<1> &G, uint32_t (&r)[L], c
 #pragma unroll
   for (int k = 0; k < L; k++) r[k] = s[k];
 #pragma unroll
-  for (int i = 0; i < L; i++) redc_row<1, L>(G, r, c0, c1, n, np0, s[L + i]);
+  for (int i = 0; i < L; i++) redc_row<L>(r, c0, c1, n, np0, s[L + i]);
   // (r, c0) = (T + QN) / R < 2R: an overflow past R is removed by subtracting N
   dsub<1, L>(G, r, n, 0u - c0);
 }
@@ -97,8 +95,8 @@ __device__ __forceinline__ void mont_sqr1(const Group<1> &G, uint32_t (&r)[L], c
 // 2 A_g A_{g+T/2 mod T} that falls to it (lanes g < T/2 take their own low half against all of the partner's
 // words, lanes g >= T/2 all of their own words against the partner's high half).  Block ids per lane: 0 S lo,
 // 1 S hi, 2r and 2r + 1 the low and high blocks of P_r, T and T + 1 those of Q.  The functions say where each
-// block belongs; no kernel squares over several lanes at present (limbs: 4 x 8 was 5.7% faster than a general
-// product and gave way to the digit kernels; digits: see powm_dig_sqr).
+// block belongs.  No kernel calls them (limbs: 4 x 8 was 5.7% faster than a general product and gave way to the
+// digit kernels; digits: see powm_dig_sqr); the decomposition is kept with the test that proves it.
 
 // T-word offset of block `id` of lane g (T lanes, L limbs each).
 __host__ __device__ constexpr int sqr_block_offset(int T, int L, int g, int id) {

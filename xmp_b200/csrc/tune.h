@@ -14,14 +14,14 @@ namespace xmpb {
 constexpr int kCand = XMP_TUNE_CANDIDATES;
 constexpr int kPowmDists = 7;          // per-thread, 2, 4, 8, 16, 32 lanes, digit-serial
 constexpr int kPowmWindows = 6;        // W = 1..6
-constexpr int kElemSlots = 8;          // {register, streamed} x {32, 64, 128, 256} threads
+constexpr int kElemSlots = 8;          // {register, other} x {32, 64, 128, 256} threads
 constexpr int kGridMaxLimbs = 512;     // selector lookup grid: precisions 32..16384 bits
 constexpr int kGridCountBuckets = 27;  // floor(log2 count), 0..26
 constexpr int kGridExpBuckets = 15;    // floor(log2 exp_bits), 0..14 (powm only)
 constexpr int kSelectorMinCountLog2 = 6;  // smallest batch the tuner times (2^6); smaller batches use its cell
 
 struct ElemConfig {
-  int variant = 0;   // 0 register kernel, 1 streamed kernel
+  int variant = 0;   // 0 register kernel, 1 lane kernel (above 512 limbs: streamed)
   int threads = 128;
 };
 

@@ -118,7 +118,7 @@ bool tuner_lookup_powm(xmpHandle_t h, uint32_t nlimbs, uint32_t exp_bits, uint32
     // A cell of the table stands for all counts between two powers of two, by their middle, and the number of
     // warps on the fullest scheduler steps inside it.  So the next cells' kernels are asked too, and the one that
     // the cost model puts 8% or more below the cell's own is taken (smaller differences are left to the
-    // network).  Mean regret on the 409 measured powm shapes 1.01 -> 0.76%; 3072 bits x 2,001: 28.1 ms on the
+    // network).  Mean regret of the table's choices on the 409 measured powm shapes 1.01 -> 0.76%; 3072 bits x 2,001: 28.1 ms on the
     // cell's 16 lanes, 25 on 8; 512 bits x 4,283: 677 us on one lane, 624 on 4.
     if (cfg->dist == kDistLanes) {
       double best = powm_shape_cycles(cfg->tpi, cfg->limbs, count, h->sm_count) / 1.08;
@@ -138,7 +138,8 @@ bool tuner_lookup_powm(xmpHandle_t h, uint32_t nlimbs, uint32_t exp_bits, uint32
     // The selector's window, kept within one of the analytic rule's (the network has seen exponents of
     // 17, 256, 1024 bits and the full precisions; the bound keeps it from straying elsewhere); the rule
     // alone where it wants a window beyond the six the tuner times.  On the committed B200 dataset this
-    // lowers the mean regret on all 409 powm shapes from 0.87% to 0.58% (held-out ones 1.51 -> 1.41%).
+    // lowers the mean regret of the networks' choices, asked at each shape itself rather than through the
+    // table, on all 409 powm shapes from 0.87% to 0.58% (held-out ones 1.51 -> 1.41%).
     const int wa = window_for_bits(exp_bits, cfg->dist != kDistDigit && powm_sliding(cfg->tpi, cfg->limbs));
     cfg->window = wa > 6 ? wa : std::max(wa - 1, std::min(wa + 1, cfg->window));
   }
