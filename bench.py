@@ -12,10 +12,12 @@ exponent.  Metric: 2048-bit modexp/s (higher is better).
             per step, xmpIntegersImport of base/exp/mod from pinned host memory,
             xmpIntegersPowm, xmpIntegersExport of the result to pinned host
             memory, all inside the timed region.
-  roofline -- the powm kernel's algorithmic INT32 multiply-adds per launch
-            (k + ceil(k/5)) * (4n^2 + n) per modexp, n = 64 limbs, k = 2048,
-            over its event-timed duration, against the IMAD peak measured live
-            by libxmpprobe.so on the same device.
+  roofline -- the FP64 operations of the powm kernel's digit products per launch
+            (three a product of 52-bit digits, 2 N^2 of those a Montgomery
+            product, N = 40 digits at 2048 bits, and k + k/(W+1) + 2^(W-1)
+            products per modexp), over its event-timed duration, against the
+            FP64 rate measured live by libxmpprobe.so on the same device.  A
+            kernel on 32-bit limbs: its multiply-adds against the IMAD rate.
   cpu_baseline -- GMP mpz_powm on the host's cores (OpenMP) on a bounded
             sample of the same instances (the oracle, as the reference's own
             perf harness compares against GMP, perf_tests/main.cu:153-229).
@@ -50,6 +52,20 @@ L2_BYTES = 126 * 1024 * 1024
 def imad_per_modexp(bits, ebits):
     n = bits // 32
     return (ebits + math.ceil(ebits / 5)) * (4 * n * n + n)
+
+
+def powm_roofline(cfg, bits, ebits, count, ms, peaks):
+    """The pipe that the products of the lane kernel `cfg` run on: achieved and peak operations."""
+    if cfg.distribution != 0 or cfg.limbs < 6:  # 32-bit limbs, or one instance per CTA
+        bound, unit, ops = "imad", "TIMAD/s", imad_per_modexp(bits, ebits)
+    else:
+        n = cfg.lanes * math.ceil((32 * cfg.lanes * cfg.limbs + 2) / (52 * cfg.lanes))  # digits, R >= 4 N
+        extra = math.ceil(ebits / (cfg.window + 1)) + 2 ** (cfg.window - 1)
+        square = n * (n + 1) // 2 + n * n if cfg.lanes == 1 else 2 * n * n
+        bound, unit, ops = "fp64", "T FP64 operations/s", 3 * (ebits * square + extra * 2 * n * n)
+    achieved = ops * count / (ms * 1e-3) / 1e12
+    return {"bound": bound, "achieved": achieved, "peak": peaks[bound], "unit": unit, "frac": achieved / peaks[bound],
+            "operations_per_modexp": ops}
 
 
 def replica_seed(rank):
@@ -134,29 +150,30 @@ class ClockSampler:
                 "reasons": sorted(reasons), "samples": len(sm)}
 
 
-def profiled_traffic(bits, count):
-    """DRAM bytes per powm launch from a committed ncu capture of this exact workload
+def profiled_traffic(bits, count, cfg):
+    """DRAM bytes per powm launch from a committed ncu capture of this exact workload on this very kernel
     (dram__bytes_read.sum + dram__bytes_write.sum), or None."""
     try:
         with open(os.path.join(ROOT, "profiles", "powm_kernel_%dbit_traffic.json" % bits)) as f:
             d = json.load(f)
     except (OSError, ValueError):
         return None
-    return d.get("dram_bytes_per_launch") if d.get("instances") == count else None
+    same = d.get("instances") == count and d.get("kernel") == [cfg.lanes, cfg.limbs, cfg.window]
+    return d.get("dram_bytes_per_launch") if same else None
 
 
-def probe_imad_peak():
+def probe_peaks():
     lib = ctypes.CDLL(os.path.join(ROOT, "xmp_b200", "libxmpprobe.so"))
     lib.xmpb_probe_imad.argtypes = [ctypes.c_int, ctypes.c_int, ctypes.c_int, ctypes.POINTER(ctypes.c_double),
                                     ctypes.POINTER(ctypes.c_double)]
     res = {}
-    for mode, name in ((0, "imad"), (1, "carry_rows")):
+    for mode, name in ((0, "imad"), (1, "carry_rows"), (2, "fp64")):
         best = 0.0
         for _ in range(3):
             imads, ms = ctypes.c_double(), ctypes.c_double()
             rc = lib.xmpb_probe_imad(mode, 8, 2048, ctypes.byref(imads), ctypes.byref(ms))
             if rc != 0:
-                raise RuntimeError("IMAD probe failed with CUDA error %d" % rc)
+                raise RuntimeError("throughput probe failed with CUDA error %d" % rc)
             best = max(best, imads.value / (ms.value * 1e-3))
         res[name] = best / 1e12
     return res
@@ -234,9 +251,9 @@ def powm_rows(h, x, e, m):
             v.destroy()
 
 
-def config1_suite(h, stream, flush, steps, warmup, imad_peak, cpu_seconds):
+def config1_suite(h, stream, flush, steps, warmup, peaks, cpu_seconds):
     """Plain batched powm, 4,096 independent 1024-bit instances with full-length exponents
-    (seeded like the headline): device-resident modexp/s, IMAD roofline, end to end through
+    (seeded like the headline): device-resident modexp/s, roofline, end to end through
     the C API with pinned host buffers, GMP on the host, every result checked against GMP."""
     import torch
     import oracle as orc
@@ -271,12 +288,10 @@ def config1_suite(h, stream, flush, steps, warmup, imad_peak, cpu_seconds):
     rate, used, sample, dt = cpu_gmp_rate(x, e, m, target_s=cpu_seconds)
     for v in (X, E, M, O):
         v.destroy()
-    achieved = imad_per_modexp(bits, bits) * count / (ms * 1e-3) / 1e12
     return {"workload": "batched powm 1024-bit x 4096 instances, full-length exponents",
             "value": count / (ms * 1e-3), "unit": "modexp/s", "ms_per_step": ms,
             "kernel": {"lanes": cfg.lanes, "limbs": cfg.limbs, "window": cfg.window},
-            "roofline": {"bound": "imad", "achieved": achieved, "peak": imad_peak, "unit": "TIMAD/s",
-                         "frac": achieved / imad_peak},
+            "roofline": powm_roofline(cfg, bits, bits, count, ms, peaks),
             "e2e": {"value": count / (e2e_ms * 1e-3), "unit": "modexp/s", "h2d_bytes_per_step": 3 * count * n * 4,
                     "d2h_bytes_per_step": count * n * 4},
             "cpu_baseline": {"value": rate, "unit": "modexp/s", "cores": used, "kind": "port",
@@ -284,9 +299,9 @@ def config1_suite(h, stream, flush, steps, warmup, imad_peak, cpu_seconds):
             "result_check": ok}
 
 
-def sweep_suite(h, stream, flush, imad_peak, counts=(4096, 16384, 65536, 262144), steps=3):
+def sweep_suite(h, stream, flush, peaks, counts=(4096, 16384, 65536, 262144), steps=3):
     """The 2048-bit workload (full-length exponents) over batch sizes 2^12 .. 2^18: modexp/s and the
-    IMAD roofline fraction per size with the library's default choice, 32 results per size checked
+    roofline fraction per size with the library's default choice, 32 results per size checked
     against GMP."""
     import oracle as orc
     import xmp_b200 as xmp
@@ -302,8 +317,9 @@ def sweep_suite(h, stream, flush, imad_peak, counts=(4096, 16384, 65536, 262144)
         ms = statistics.median(_timed_events(step, stream, flush, steps, 1))
         want, _ = orc.powm(x[:32], e[:32], m[:32], 32)
         ok = bool(np.array_equal(O.export()[:32], want))
-        achieved = imad_per_modexp(bits, bits) * count / (ms * 1e-3) / 1e12
-        out[str(count)] = {"value": count / (ms * 1e-3), "unit": "modexp/s", "ms": ms, "imad_frac": achieved / imad_peak,
+        roof = powm_roofline(cfg, bits, bits, count, ms, peaks)
+        out[str(count)] = {"value": count / (ms * 1e-3), "unit": "modexp/s", "ms": ms, "bound": roof["bound"],
+                           "frac": roof["frac"],
                            "kernel": {"distribution": cfg.distribution, "lanes": cfg.lanes, "limbs": cfg.limbs,
                                       "window": cfg.window}, "check": ok}
         for v in (X, E, M, O):
@@ -485,15 +501,12 @@ def run_ours(args, rank, world, local_rank):
 
     if rank != 0:
         return
-    peaks = probe_imad_peak()
-    algo = imad_per_modexp(bits, bits) * count  # per launch
-    kernel_s = statistics.median(step_ms) * 1e-3
-    achieved = algo / kernel_s / 1e12
-    roofline = {"bound": "imad", "achieved": achieved, "peak": peaks["imad"], "unit": "TIMAD/s",
-                "frac": achieved / peaks["imad"], "traffic": profiled_traffic(bits, count),
-                "peak_source": "measured live: libxmpprobe independent mad.lo.u32 chains, all SMs",
-                "carry_row_peak": peaks["carry_rows"],
-                "algorithmic_imad_per_modexp": imad_per_modexp(bits, bits)}
+    peaks = probe_peaks()
+    cfg = forced or xmp.powm_get_config(h, bits, bits, count)
+    roofline = powm_roofline(cfg, bits, bits, count, statistics.median(step_ms), peaks)
+    roofline["traffic"] = profiled_traffic(bits, count, cfg)
+    roofline["peak_source"] = "measured live: libxmpprobe independent %s chains, all SMs" % (
+        "fma.rz.f64" if roofline["bound"] == "fp64" else "mad.lo.u32")
 
     cpu = None
     if not args.no_cpu:
@@ -511,7 +524,7 @@ def run_ours(args, rank, world, local_rank):
         # the other single-GPU workloads, measured after the headline's timed regions (rank 0, N = 1)
         t0 = time.perf_counter()
         extra = {}
-        extra["config1_1024bit_x4096"] = config1_suite(h, stream, flush, args.steps, args.warmup, peaks["imad"],
+        extra["config1_1024bit_x4096"] = config1_suite(h, stream, flush, args.steps, args.warmup, peaks,
                                                        min(args.cpu_seconds, 3.0))
         xx, ee, mm = make_inputs(1024, 4096)
         ours1 = {(bits, count): res.copy(), (1024, 4096): powm_rows(h, xx, ee, mm)}
@@ -521,7 +534,7 @@ def run_ours(args, rank, world, local_rank):
                                         "imad_peak_timad_s": peaks["imad"]}
         extra["config3_mixed"] = mixed_suite(3, 1, 65536, 16384, 256)
         extra["single_op_latency"] = latency_suite(h, stream)
-        extra["powm2048_batch_sweep"] = sweep_suite(h, stream, flush, peaks["imad"])
+        extra["powm2048_batch_sweep"] = sweep_suite(h, stream, flush, peaks)
         extra["config5_serving"] = serving_quick()
         extra["seconds"] = time.perf_counter() - t0
 
@@ -1003,7 +1016,7 @@ def run_elementwise(args):
     h = xmp.Handle()
     stream = torch.cuda.current_stream()
     h.set_stream(stream.cuda_stream)
-    imad_peak = probe_imad_peak()["imad"]
+    imad_peak = probe_peaks()["imad"]
     res, cpu, hbm = elementwise_suite(h, stream, args.steps, args.warmup, imad_peak)
     line = {"metric": "elementwise suite HBM GB/s (256-bit add)", "value": res["add"]["gbs"], "unit": "GB/s",
             "higher_is_better": True, "n_gpus": 1, "steps": args.steps, "warmup": args.warmup,

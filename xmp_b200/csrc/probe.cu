@@ -1,8 +1,10 @@
-// INT32 multiply-add throughput microbenchmark (libxmpprobe.so): measures the
-// roofline denominator for the integer kernels on the device it runs on.
+// Multiply-add throughput microbenchmark (libxmpprobe.so): measures the roofline
+// denominators for the integer and the digit kernels on the device it runs on.
 //   mode 0: independent mad.lo.u32 chains (plain IMAD issue rate)
 //   mode 1: mad.lo.cc / madc.hi.cc carry-chain rows shaped like the Montgomery
 //           inner loop (2L multiply-adds + 2 carry adds per row, L = 8)
+//   mode 2: independent fma.rz.f64 chains (plain FP64 issue rate, the digit
+//           products' pipe)
 // Every instruction is inline PTX so the count per thread is exact; the
 // result is written out so nothing is dead.
 #include <cuda_runtime.h>
@@ -64,6 +66,24 @@ __global__ void __launch_bounds__(256) imad_rows(uint32_t *out, int iters, uint3
   out[blockIdx.x * blockDim.x + threadIdx.x] = s;
 }
 
+__global__ void __launch_bounds__(256) fp64_plain(uint32_t *out, int iters, uint32_t seed) {
+  double a[8];
+  const double b = 0.5 + seed * 0x1p-40, c = 1.0 + threadIdx.x * 0x1p-30;  // the chains stay near 2
+#pragma unroll
+  for (int k = 0; k < 8; k++) a[k] = k;
+  for (int i = 0; i < iters; i++) {
+#pragma unroll
+    for (int u = 0; u < 8; u++) {
+#pragma unroll
+      for (int k = 0; k < 8; k++) asm volatile("fma.rz.f64 %0, %0, %1, %2;" : "+d"(a[k]) : "d"(b), "d"(c));
+    }
+  }
+  double s = 0;
+#pragma unroll
+  for (int k = 0; k < 8; k++) s += a[k];
+  out[blockIdx.x * blockDim.x + threadIdx.x] = __double2loint(s);
+}
+
 PROBE_API int xmpb_probe_imad(int mode, int blocks_per_sm, int iters, double *imads, double *ms) {
   int dev = 0, sms = 0;
   cudaGetDevice(&dev);
@@ -78,6 +98,7 @@ PROBE_API int xmpb_probe_imad(int mode, int blocks_per_sm, int iters, double *im
   auto launch = [&](int it) {
     switch (mode) {
       case 0: imad_plain<<<blocks, threads>>>(out, it, 12345u); break;
+      case 2: fp64_plain<<<blocks, threads>>>(out, it, 12345u); break;
       default: imad_rows<<<blocks, threads>>>(out, it, 12345u); break;
     }
   };
@@ -89,7 +110,7 @@ PROBE_API int xmpb_probe_imad(int mode, int blocks_per_sm, int iters, double *im
   float f = 0;
   cudaEventElapsedTime(&f, t0, t1);
   *ms = f;
-  // multiply-adds per thread per iteration (both modes: 64)
+  // multiply-adds per thread per iteration (every mode: 64)
   *imads = (double)blocks * threads * iters * 64.0;
   cudaEventDestroy(t0);
   cudaEventDestroy(t1);
