@@ -39,7 +39,8 @@ xmpError_t XMPAPI xmpPowmKernelCount(int32_t *count);
 xmpError_t XMPAPI xmpPowmKernelGet(int32_t index, int32_t *lanes, int32_t *limbs);
 
 /* The configuration xmpIntegersPowm would use now for this problem shape
- * (tuned entry if the handle's tuner has one, else the built-in heuristic). */
+ * under the handle's policy: a choice set for the exact shape, else one instance
+ * per CTA for small batches, else the selector, else the built-in heuristic. */
 xmpError_t XMPAPI xmpPowmGetConfig(xmpHandle_t handle, uint32_t precision, uint32_t exp_precision, uint32_t count,
                                    xmpPowmConfig_t *config);
 
@@ -57,8 +58,9 @@ xmpError_t XMPAPI xmpIntegersPowmWithConfigAsync(xmpHandle_t handle, xmpIntegers
  * out = mq + q * ((mp - mq) * qinv mod p), Garner recombination; p and q
  * have their top bit set).  Instances are binned by modulus precision (CRT
  * halves join the bin of their precision); every bin runs as one persistent
- * kernel whose warps pull work from an atomic queue, with its configuration
- * from the handle's tuner, and all bins run concurrently (forked onto side
+ * kernel whose warps pull work from an atomic queue, with a choice set for the
+ * exact shape or else the kernel that the library's cost model expects to take
+ * the bin through soonest, and all bins run concurrently (forked onto side
  * streams and joined back to the handle's stream).  With `use_graph` the
  * whole execution is captured once into a CUDA graph and each execute is one
  * graph launch.  All device memory a plan needs (window tables, CRT

@@ -12,10 +12,11 @@
 // registers (BN limbs, a compile-time class) together with a BN+1 limb window
 // of the partial remainder.  The shifted dividend is never materialised: each
 // step pulls its next limb straight from the interleaved input with the
-// funnel shift applied.  The quotient digit estimate divides the top two
-// window limbs by the top divisor limb with a precomputed reciprocal
+// funnel shift applied.  The quotient digit estimate divides the top three
+// window limbs by the top two divisor limbs with a precomputed reciprocal
 // (Moller & Granlund, "Improved division by invariant integers", IEEE TC
-// 2011, algorithm 4), refined once against the second divisor limb; the
+// 2011, algorithm 5; one-limb divisors and the scratch kernel: algorithm 4,
+// two limbs by one, refined against the second divisor limb); the
 // multiply-subtract then needs at most one add-back.
 // Larger divisors (up to 512 limbs) spread divisor and window over the lanes of
 // a group; beyond that the same algorithm keeps them in the scratch arena.

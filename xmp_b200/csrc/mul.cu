@@ -6,9 +6,10 @@
 // Register path: the larger operand is held in registers as AL limbs, the
 // smaller as BL limbs (AL, BL from a small set of classes), and the AL+BL-limb
 // product is formed by operand scanning, one row of two mad chains (low and
-// high halves) per limb of the smaller operand.  Large path (either operand
-// above 32 limbs): product scanning straight from the interleaved arrays with
-// a three-word column accumulator, so nothing has to fit in registers.
+// high halves) per limb of the smaller operand.  Above 32 limbs: the larger
+// operand spread over the lanes of a group, up to 512 limbs; beyond, and for an
+// explicit digit-serial algorithm, product scanning straight from the
+// interleaved arrays with a three-word column accumulator.
 // Squaring (a == b without index arrays, src/mul.cu:147-149) takes the same
 // kernels.
 #include "internal.h"
